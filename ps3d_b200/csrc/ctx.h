@@ -227,6 +227,7 @@ struct Ctx {
 
     int init(const ps3d_params& prm, int dev, int nbatch = 1, cudaStream_t use_stream = nullptr);
     int autotune();
+    int model_kchunk() const;   // the step kernel's z chunk by the wave model (engine.cu)
     int advance(int nsteps, bool allow_graph);
     bool graphable() const;
     int capture_graph(GraphSlot& slot);

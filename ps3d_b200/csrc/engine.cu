@@ -415,7 +415,7 @@ int Ctx::init(const ps3d_params& prm, int dev, int nbatch, cudaStream_t use_stre
     *kerr_h = 0;
     CK(cudaHostGetDevicePointer((void**)&kerr_d, kerr_h, 0));
     pa64.err = kerr_d; pa32.err = kerr_d;
-    kchunk = nz <= 16 ? nz : 8;
+    kchunk = model_kchunk();
     // reductions
     nred = 148 * 4;
     CK(red_partials.alloc((size_t)nred * 5 * sizeof(double)));
@@ -658,6 +658,31 @@ static void tune_cache_store(const std::string& k, const std::string& v) {
     }
 }
 
+// The step kernel's z chunk that minimises waves x (levels + 3): a block's
+// fixed part (launch, three planes of latency and their correction) costs
+// about three levels of its march (measured 6.5 us + 1.25 us a level at
+// 32x32x16), and a last wave that is nearly empty costs a whole one.  At
+// 32x32x16 it gives 1 (64 blocks, 7.5 us; 34 us as one chunk of 16), at
+// 64x64x32 2, at 256x256x128 12 (6.3 waves of 444 blocks).
+int Ctx::model_kchunk() const {
+    StepArgs q{};
+    q.harm_uvw = (P.Ah > 0. || P.Av > 0.); q.harm_b = (P.Kh > 0. || P.Kv > 0.);
+    q.wm_on = (fkind & PS3D_FORCE_WAVEMAKER) ? 1 : 0;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const long slots = (long)sms * step_resident(q, hist32);
+    const long tiles = (long)((nx + 31) / 32) * ((ny + 7) / 8) * std::max(1, batch);
+    const int levels = win_kcount ? win_kcount : nz;
+    double bestc = 1e300;
+    int best = 1;
+    for (int kc = 1; kc <= std::min(levels, 48); ++kc) {
+        const long blocks = tiles * ((levels + kc - 1) / kc);
+        const double c = (double)((blocks + slots - 1) / slots) * (kc + 3);
+        if (c < bestc * (1 - 1e-9)) { bestc = c; best = kc; }
+    }
+    return best;
+}
+
 int Ctx::autotune() {
     std::lock_guard<std::mutex> tune_lock(g_tune_mu);
     const char* env = std::getenv("PS3D_AUTOTUNE");
@@ -669,7 +694,7 @@ int Ctx::autotune() {
     cudaDeviceProp prop;
     CK(cudaGetDeviceProperties(&prop, dev));
     char key[384];
-    std::snprintf(key, sizeof key, "%s|%dx%dx%d|p%d|r%d|b%d|i%d", prop.name, nx, ny, nz, (int)mixed, (int)rigid, batch,
+    std::snprintf(key, sizeof key, "%s|%dx%dx%d|p%d|r%d|b%d|i%d|s2", prop.name, nx, ny, nz, (int)mixed, (int)rigid, batch,
                   plane_force);
     for (char* c = key; *c; ++c) if (*c == ' ') *c = '_';
     const bool f32 = mixed;
@@ -757,30 +782,16 @@ int Ctx::autotune() {
     }
     bestpa.batch = 1;
     pa = bestpa;
-    // step kernel z chunk: 4, 8, 16, 32 and the chunk that best fills the
-    // last wave of blocks (cost ~ waves x (kc + 2) plane loads per block:
-    // at 256x256x128, kc 15 gives 2304 blocks, 3.9 waves of 592, against
-    // kc 16's 2048 blocks, 3.5 waves: 308 against 314 us)
-    std::vector<int> kcs = {4, 8, 16, 32};
+    // step kernel z chunk: powers of two and the chunk of the wave model
+    std::vector<int> kcs = {1, 2, 4, 8, 16, 32};
     {
-        StepArgs q{};
-        q.harm_uvw = (P.Ah > 0. || P.Av > 0.); q.harm_b = (P.Kh > 0. || P.Kv > 0.);
-        q.wm_on = (fkind & PS3D_FORCE_WAVEMAKER) ? 1 : 0;
-        const long slots = (long)prop.multiProcessorCount * step_resident(q, hist32);
-        const long tiles = (long)((nx + 31) / 32) * ((ny + 7) / 8) * std::max(1, batch);
-        double bestc = 1e300;
-        int mkc = 16;
-        for (int kc = 4; kc <= std::min(nz, 48); ++kc) {
-            const long blocks = tiles * ((nz + kc - 1) / kc);
-            const double c = (double)((blocks + slots - 1) / slots) * (kc + 2);
-            if (c < bestc * (1 - 1e-9)) { bestc = c; mkc = kc; }
-        }
+        const int mkc = model_kchunk();
         if (std::find(kcs.begin(), kcs.end(), mkc) == kcs.end()) kcs.push_back(mkc);
     }
     float bestk = 1e30f;
     int bestkc = kchunk;
     for (int kc : kcs) {
-        if (kc > nz) continue;
+        if (kc > nz || (long)((nz + kc - 1) / kc) * batch > 65535) continue;   // beyond the launch grid's z limit
         kchunk = kc;
         const float t = timeit([&]() -> int {
             StepArgs a{};

@@ -11,217 +11,88 @@
 //   set_forcing (wavemaker and
 //     background-flow advection)      config.f90:224-237, lee_wave1.f90:232-332
 //   Adams-Bashforth 2/3               integrate.f90:87-102
-// The block owns a 32 x BY column tile and marches up in z; the three planes
-// k-1, k, k+1 of u, v, w, b (and of U_back, B_back when present) sit in a
-// shared-memory ring with a one-point halo.  Each thread's tile elements and
-// their east/north neighbours are located once per block, so a plane load is
-// one offset add per field.  Face fluxes are recomputed per
-// point instead of being stored, so the kernel reads each state word once
-// from HBM and writes tendencies and the new state once.
+// The block owns a 32 x BY column tile and marches up in z, two neighbouring
+// points along x per thread.  Levels k and k+1 of u, v, w, b (and of U_back,
+// B_back when present) sit corrected in a four-slot shared-memory ring; level
+// k+2 has landed and gets its pending pressure correction while level k is
+// stepped, and level k+3 is on its way (16-byte asynchronous copies), so one
+// barrier a level is enough and no load is waited for where it is issued.  The
+// vertical fluxes and a column's own values pass from level to level in
+// registers; only the level's horizontal neighbours are read from the ring.
+// Each state word is read once from HBM and each tendency and new value is
+// written once.
+//
+// What bounds it: HBM.  At 256x256x128 it runs 237 us in FP64 (168 B a point,
+// 5.9 TB/s) and 222-231 us in the mixed form (132 B, 4.9 TB/s).  The form it
+// replaced (one point a thread, planes loaded through registers behind two
+// barriers a level, all fluxes formed from shared memory) took 321 and 292 us:
+// it kept the L1/shared data path at 72 % with 257 wavefronts and 632
+// instructions per 32 points, against 140 and 365 now.
 #include <cstdlib>
+#include <type_traits>
 #include "engine.h"
 
 namespace ps3d {
 
 constexpr int kTX = 32;
 
-// The ring of state planes, and this level's Adams-Bashforth history of the
-// block's points (t1, t2), staged through shared memory so that its loads
-// go out with the next plane's before the barrier without holding
-// registers through the tendency arithmetic.
+// The ring of state planes, filled by 16-byte asynchronous copies three
+// levels ahead of the level that is stepped: levels k and k+1 (corrected,
+// read by the stencil), k+2 (landed, being corrected) and k+3 (on its way).
+// Tiles start two columns west of the block's first point so that every
+// 16-byte pair is aligned (nx is even: a pair never straddles the periodic
+// seam); the pressure tile has one row and one pair more, for the
+// correction's north and east neighbours.  The level's Adams-Bashforth
+// history is copied to a slot of the thread's own.
+template <int BY>
+struct StepTile {
+    static constexpr int NT = kTX / 2 * BY;           // threads: a pair of points along x each
+    static constexpr int FP = kTX + 4, FR = BY + 2;   // field tile: columns i0-2 .. i0+33, rows j0-1 .. j0+BY
+    static constexpr int PP = kTX + 6, PR = BY + 3;   // pressure tile: columns i0-2 .. i0+35, rows j0-1 .. j0+BY+1
+    static constexpr int FCH = FP / 2 * FR, PCH = PP / 2 * PR;   // pairs of a tile
+};
+template <typename TT> struct pair_t;
+template <> struct pair_t<double> { using type = double2; };
+template <> struct pair_t<float> { using type = float2; };
+
 template <typename TT, int BY, int NF>
-struct StepSmem {
-    double pl[NF][3][(BY + 2) * (kTX + 2)];
-    TT hu[2][kTX * BY], hv[2][kTX * BY], hb[2][kTX * BY];
-    double hw[2][kTX * BY];
+struct __align__(16) StepSmem {
+    double pl[4][NF][StepTile<BY>::FP * StepTile<BY>::FR];
+    double pp[4][StepTile<BY>::PP * StepTile<BY>::PR];
+    double2 hw[2][StepTile<BY>::NT];
+    typename pair_t<TT>::type hist[2][3][StepTile<BY>::NT];   // u, v, b
 };
 
-// The tendency, friction, forcing and Adams-Bashforth update of the point
-// (i, j, k) of instance `ioff`: F(f, di, dj, dk) reads field f (0 u, 1 v,
-// 2 w, 3 b, 4 U_back, 5 B_back) of the corrected state at the offsets,
-// Hh(f, l) the point's stored tendency of field f at history level l
-// (0: taum1, 1: taum2).  Shared by the step kernels, which differ only in
-// how they stage the state.
-template <typename TT, bool HARM, bool WM, bool BG, class FV, class HV>
-__device__ __forceinline__ void step_point(const StepArgs& a, const FV& F, const HV& Hh, int i, int j, int k,
-                                           long ioff, bool h1, bool h2) {
-    using TW = double;   // stored w tendencies stay FP64 in both paths
-    const int nx = a.nx, ny = a.ny;
-    const long plane = (long)nx * ny;
-    const int kofs = a.kofs, nzg = a.nzg ? a.nzg : a.nz;
-    const double Ro = a.Ro, rdx = a.rdx, rdy = a.rdy, rdz = a.rdz;
-    const bool rigid = a.rigid;
-#define U(di, dj, dk) F(0, di, dj, dk)
-#define V(di, dj, dk) F(1, di, dj, dk)
-#define W(di, dj, dk) F(2, di, dj, dk)
-#define B(di, dj, dk) F(3, di, dj, dk)
-#define UB(di, dj, dk) F(4, di, dj, dk)
-#define BB(di, dj, dk) F(5, di, dj, dk)
-    const int kg = k + kofs;                     // global level
-    const bool top = rigid && (kg == nzg - 1);   // flux_top(nz) = 0
-    const bool bot = rigid && (kg == 0);         // flux_top(0)  = 0
-    const long g0 = (long)k * plane + (long)j * nx + i;   // point within the instance
-    const long g = g0 + ioff;                              // point within the batch
-    double db_, du_, dv_, dw_;
-    // ---- buoyancy advection + N^2 (advection.f90:12-47, integrate.f90:21-23)
-    // The reference's 0.5 and 0.25 flux factors are powers of two: they
-    // are carried in the per-axis factors a.hd* = 0.5/d*, a.qd* = 0.25/d*
-    // (and 0.25 f0, 0.5 N0^2, set by the launcher), a multiply saved per
-    // flux.  Scaling by a power of two rounds exactly; the results move
-    // at round-off level only where the compiler now contracts a flux
-    // product into the difference that follows (FMA).
-    if (a.nonlinear) {
-        const double fe = (B(0, 0, 0) + B(1, 0, 0)) * U(0, 0, 0);
-        const double fem = (B(-1, 0, 0) + B(0, 0, 0)) * U(-1, 0, 0);
-        const double fn = (B(0, 0, 0) + B(0, 1, 0)) * V(0, 0, 0);
-        const double fnm = (B(0, -1, 0) + B(0, 0, 0)) * V(0, -1, 0);
-        const double ft = top ? 0.0 : (B(0, 0, 0) + B(0, 0, 1)) * W(0, 0, 0);
-        const double ftm = bot ? 0.0 : (B(0, 0, -1) + B(0, 0, 0)) * W(0, 0, -1);
-        db_ = -Ro * ((fe - fem) * a.hdx + (fn - fnm) * a.hdy + (ft - ftm) * a.hdz);
-        // ---- zonal momentum (advection.f90:65-100)
-        {
-            const double e = (U(0, 0, 0) + U(1, 0, 0)) * (U(1, 0, 0) + U(0, 0, 0));
-            const double em = (U(-1, 0, 0) + U(0, 0, 0)) * (U(0, 0, 0) + U(-1, 0, 0));
-            const double n = (U(0, 0, 0) + U(0, 1, 0)) * (V(1, 0, 0) + V(0, 0, 0));
-            const double nm = (U(0, -1, 0) + U(0, 0, 0)) * (V(1, -1, 0) + V(0, -1, 0));
-            const double t = top ? 0.0 : (U(0, 0, 1) + U(0, 0, 0)) * (W(0, 0, 0) + W(1, 0, 0));
-            const double tm = bot ? 0.0 : (U(0, 0, 0) + U(0, 0, -1)) * (W(0, 0, -1) + W(1, 0, -1));
-            du_ = -Ro * ((e - em) * a.qdx + (n - nm) * a.qdy + (t - tm) * a.qdz);
-        }
-        // ---- meridional momentum (advection.f90:104-140)
-        {
-            const double e = (V(0, 0, 0) + V(1, 0, 0)) * (U(0, 1, 0) + U(0, 0, 0));
-            const double em = (V(-1, 0, 0) + V(0, 0, 0)) * (U(-1, 1, 0) + U(-1, 0, 0));
-            const double n = (V(0, 0, 0) + V(0, 1, 0)) * (V(0, 1, 0) + V(0, 0, 0));
-            const double nm = (V(0, -1, 0) + V(0, 0, 0)) * (V(0, 0, 0) + V(0, -1, 0));
-            const double t = top ? 0.0 : (V(0, 0, 1) + V(0, 0, 0)) * (W(0, 0, 0) + W(0, 1, 0));
-            const double tm = bot ? 0.0 : (V(0, 0, 0) + V(0, 0, -1)) * (W(0, 0, -1) + W(0, 1, -1));
-            dv_ = -Ro * ((e - em) * a.qdx + (n - nm) * a.qdy + (t - tm) * a.qdz);
-        }
-        // ---- vertical momentum (advection.f90:145-181); rigid lid zeroes
-        //      flux_top(nz-1:nz+2) for w (:167-170)
-        {
-            const bool wtop = rigid && (kg >= nzg - 2);
-            const bool wbot = rigid && (kg == 0 || kg >= nzg - 1);
-            const double e = (W(0, 0, 0) + W(1, 0, 0)) * (U(0, 0, 0) + U(0, 0, 1));
-            const double em = (W(-1, 0, 0) + W(0, 0, 0)) * (U(-1, 0, 0) + U(-1, 0, 1));
-            const double n = (W(0, 0, 0) + W(0, 1, 0)) * (V(0, 0, 0) + V(0, 0, 1));
-            const double nm = (W(0, -1, 0) + W(0, 0, 0)) * (V(0, -1, 0) + V(0, -1, 1));
-            const double t = wtop ? 0.0 : (W(0, 0, 1) + W(0, 0, 0)) * (W(0, 0, 0) + W(0, 0, 1));
-            const double tm = wbot ? 0.0 : (W(0, 0, 0) + W(0, 0, -1)) * (W(0, 0, -1) + W(0, 0, 0));
-            dw_ = -a.dsqr * Ro * ((e - em) * a.qdx + (n - nm) * a.qdy + (t - tm) * a.qdz);
-        }
-    } else {
-        db_ = du_ = dv_ = dw_ = 0.0;
-    }
-    db_ = db_ - (W(0, 0, 0) + W(0, 0, -1)) * a.hN0sq;
-    // ---- Coriolis, buoyancy force, rigid-lid mask (integrate.f90:37-54)
-    du_ = du_ + (V(0, 0, 0) + V(0, -1, 0) + V(1, 0, 0) + V(1, -1, 0)) * a.qf0;
-    dv_ = dv_ - (U(-1, 0, 0) + U(0, 0, 0) + U(-1, 1, 0) + U(0, 1, 0)) * a.qf0;
-    dw_ = dw_ + 0.5 * (B(0, 0, 0) + B(0, 0, 1));
-    if (top) dw_ = 0.0;
-    // ---- friction, in place before AB (integrate.f90:59-66)
-    double u1 = U(0, 0, 0), v1 = V(0, 0, 0), w1 = W(0, 0, 0), b1 = B(0, 0, 0);
-    if constexpr (HARM) {
-        const double dt = a.dt;
-#define HARMONIC(F, Hm, Vm, out)                                                                   \
-    {                                                                                            \
-const double e = Hm * (F(1, 0, 0) - F(0, 0, 0)) * rdx;                                   \
-const double em = Hm * (F(0, 0, 0) - F(-1, 0, 0)) * rdx;                                 \
-const double n = Hm * (F(0, 1, 0) - F(0, 0, 0)) * rdy;                                   \
-const double nm = Hm * (F(0, 0, 0) - F(0, -1, 0)) * rdy;                                 \
-const double t = top ? 0.0 : Vm * (F(0, 0, 1) - F(0, 0, 0)) * rdz;                       \
-const double tm = bot ? 0.0 : Vm * (F(0, 0, 0) - F(0, 0, -1)) * rdz;                     \
-out = F(0, 0, 0) + dt * ((e - em) * rdx + (n - nm) * rdy + (t - tm) * rdz);              \
-    }
-        if (a.harm_uvw) {
-            HARMONIC(U, a.Ah, a.Av, u1)
-            HARMONIC(V, a.Ah, a.Av, v1)
-            HARMONIC(W, a.Ah, a.Av, w1)
-            if (top) w1 = 0.0;
-        }
-        if (a.harm_b) HARMONIC(B, a.Kh, a.Kv, b1)
-#undef HARMONIC
-    }
-    // ---- set_forcing: background-flow advection (lee_wave1.f90:245-312)
-    if constexpr (BG) {
-        {
-            const double e = 2 * 0.25 * (UB(0, 0, 0) + UB(1, 0, 0)) * (U(1, 0, 0) + U(0, 0, 0));
-            const double em = 2 * 0.25 * (UB(-1, 0, 0) + UB(0, 0, 0)) * (U(0, 0, 0) + U(-1, 0, 0));
-            const double n = 0.25 * (UB(0, 0, 0) + UB(0, 1, 0)) * (V(1, 0, 0) + V(0, 0, 0));
-            const double nm = 0.25 * (UB(0, -1, 0) + UB(0, 0, 0)) * (V(1, -1, 0) + V(0, -1, 0));
-            const double t = top ? 0.0 : 0.25 * (UB(0, 0, 1) + UB(0, 0, 0)) * (W(0, 0, 0) + W(1, 0, 0));
-            const double tm = bot ? 0.0 : 0.25 * (UB(0, 0, 0) + UB(0, 0, -1)) * (W(0, 0, -1) + W(1, 0, -1));
-            du_ = du_ - Ro * ((e - em) * rdx + (n - nm) * rdy + (t - tm) * rdz);
-        }
-        {
-            const double e = 0.25 * (V(0, 0, 0) + V(1, 0, 0)) * (UB(0, 1, 0) + UB(0, 0, 0));
-            const double em = 0.25 * (V(-1, 0, 0) + V(0, 0, 0)) * (UB(-1, 1, 0) + UB(-1, 0, 0));
-            dv_ = dv_ - Ro * (e - em) * rdx;
-        }
-        {
-            const double e = 0.25 * (W(0, 0, 0) + W(1, 0, 0)) * (UB(0, 0, 0) + UB(0, 0, 1));
-            const double em = 0.25 * (W(-1, 0, 0) + W(0, 0, 0)) * (UB(-1, 0, 0) + UB(-1, 0, 1));
-            dw_ = dw_ - a.dsqr * Ro * (e - em) * rdx;
-        }
-        {
-            const double e = 0.5 * (B(0, 0, 0) + B(1, 0, 0)) * UB(0, 0, 0) + 0.5 * (BB(0, 0, 0) + BB(1, 0, 0)) * U(0, 0, 0);
-            const double em = 0.5 * (B(-1, 0, 0) + B(0, 0, 0)) * UB(-1, 0, 0) + 0.5 * (BB(-1, 0, 0) + BB(0, 0, 0)) * U(-1, 0, 0);
-            const double n = 0.5 * (BB(0, 0, 0) + BB(0, 1, 0)) * V(0, 0, 0);
-            const double nm = 0.5 * (BB(0, -1, 0) + BB(0, 0, 0)) * V(0, -1, 0);
-            const double t = top ? 0.0 : 0.5 * (BB(0, 0, 0) + BB(0, 0, 1)) * W(0, 0, 0);
-            const double tm = bot ? 0.0 : 0.5 * (BB(0, 0, -1) + BB(0, 0, 0)) * W(0, 0, -1);
-            db_ = db_ - Ro * ((e - em) * rdx + (n - nm) * rdy + (t - tm) * rdz);
-        }
-    }
-#undef U
-#undef V
-#undef W
-#undef B
-#undef UB
-#undef BB
-    // ---- set_forcing: wavemaker (config.f90:224-237)
-    if constexpr (WM) {
-        const double dt = a.dt, c = a.wm_c, s = a.wm_s;
-        if (a.wr[0] || a.wi[0]) u1 = u1 + dt * (c * (a.wr[0] ? a.wr[0][g0] : 0.0) + s * (a.wi[0] ? a.wi[0][g0] : 0.0));
-        if (a.wr[1] || a.wi[1]) v1 = v1 + dt * (c * (a.wr[1] ? a.wr[1][g0] : 0.0) + s * (a.wi[1] ? a.wi[1][g0] : 0.0));
-        if (a.wr[2] || a.wi[2]) w1 = w1 + dt * (c * (a.wr[2] ? a.wr[2][g0] : 0.0) + s * (a.wi[2] ? a.wi[2][g0] : 0.0));
-        if (a.wr[3] || a.wi[3]) b1 = b1 + dt * (c * (a.wr[3] ? a.wr[3][g0] : 0.0) + s * (a.wi[3] ? a.wi[3][g0] : 0.0));
-    }
-    // ---- store tendency of time level tau
-    ((TT*)a.t0[0])[g] = (TT)du_;
-    ((TT*)a.t0[1])[g] = (TT)dv_;
-    ((TW*)a.t0[2])[g] = (TW)dw_;
-    ((TT*)a.t0[3])[g] = (TT)db_;
-    // ---- Adams-Bashforth (integrate.f90:87-102)
-    if (a.do_ab) {
-        const double dt = a.dt, dtw = a.dtw;
-        const double c0 = a.ab0, c1 = a.ab1, c2 = a.ab2;
-        // the current tendency enters at full precision; only the
-        // stored history (FP32 in the mixed path) is rounded
-        double tu = c0 * du_, tv = c0 * dv_, tw = c0 * dw_, tb = c0 * db_;
-        if (h1) {
-            tu = tu + c1 * Hh(0, 0); tv = tv + c1 * Hh(1, 0);
-            tw = tw + c1 * Hh(2, 0); tb = tb + c1 * Hh(3, 0);
-        }
-        if (h2) {
-            tu = tu + c2 * Hh(0, 1); tv = tv + c2 * Hh(1, 1);
-            tw = tw + c2 * Hh(2, 1); tb = tb + c2 * Hh(3, 1);
-        }
-        u1 = u1 + dt * tu; v1 = v1 + dt * tv; w1 = w1 + dtw * tw; b1 = b1 + dt * tb;
-    }
-    a.uo[g] = u1; a.vo[g] = v1; a.wo[g] = w1; a.bo[g] = b1;
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void* dst, const void* src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(PENDING) : "memory"); }
 
-// read field f at offsets (di, dj) in ring slot s
-#define SM(fi, s, dj, di) sm.pl[fi][s][(ty + 1 + (dj)) * (kTX + 2) + (tx + 1 + (di))]
+// What a thread keeps of its two columns between two levels: its values at
+// the level (with u west and v south of them, which the fluxes through the
+// level's west and south faces have read one level earlier), the vertical
+// fluxes through the level's lower face and w below it.
+struct StepCarry {
+    double u0[2], v0[2], w0[2], b0[2], uw, vs[2];
+    double tb[2], tu[2], tv[2], tw[2];     // lower-face fluxes of b, u, v, w
+    double hu[2], hv[2], hw[2], hb[2];     // lower-face harmonic fluxes
+    double gu[2], gb[2];                   // lower-face background fluxes of u, b
+    double wm[2];
+};
 
 // One block's column tile (bx, by) and z chunk / instance bz of the grid
 // described by `a`.
-template <typename TT, int BY, bool HARM, bool WM, bool BG>
+template <typename TT, int BY, int HARM, bool WM, bool BG>
 __device__ __forceinline__ void step_tile(const StepArgs& a, int kchunk, int bx, int by, int bz) {
     using TW = double;   // stored w tendencies stay FP64 in both paths
-    constexpr int NF = BG ? 6 : 4;
+    using T2 = typename pair_t<TT>::type;
+    using L = StepTile<BY>;
+    constexpr int NF = BG ? 6 : 4, NT = L::NT;
     extern __shared__ __align__(16) unsigned char step_smem_raw[];
     StepSmem<TT, BY, NF>& sm = *reinterpret_cast<StepSmem<TT, BY, NF>*>(step_smem_raw);
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -234,92 +105,396 @@ __device__ __forceinline__ void step_tile(const StepArgs& a, int kchunk, int bx,
     const int kb = a.kbeg + (bz - inst * nzc) * kchunk;
     const int ke = min(a.kbeg + kcnt, kb + kchunk);
     const long ioff = (long)inst * a.sN;
-    const int i = i0 + tx, j = j0 + ty;
-    const bool active = (i < nx) && (j < ny);
-    const long plane = (long)nx * ny;
+    const bool active = (i0 + 2 * tx < nx) && (j0 + ty < ny);   // threads past the edge run along, storing nothing
+    const unsigned plane = (unsigned)nx * ny;
     const double* src[6] = {a.u + ioff, a.v + ioff, a.w + ioff, a.b + ioff, a.ub, a.bb};
-    const int tid = ty * kTX + tx;
-    constexpr int TP = (kTX + 2) * (BY + 2);
-
     const double* pc = a.pc ? a.pc + ioff : nullptr;
-    // per-thread tile elements: plane offsets of the point and of its east and
-    // north neighbours, computed once (full modulo: tiles may be wider than the grid)
-    constexpr int NT = kTX * BY;
-    constexpr int EPT = (TP + NT - 1) / NT;
-    int eo[EPT], eoE[EPT], eoN[EPT];
-#pragma unroll
-    for (int e = 0; e < EPT; ++e) {
-        const int t = tid + e * NT;
-        const int ti = t % (kTX + 2), tj = t / (kTX + 2);
-        const int gi = ((i0 - 1 + ti) % nx + nx) % nx, gj = ((j0 - 1 + tj) % ny + ny) % ny;
-        eo[e] = gj * nx + gi;
-        eoE[e] = gj * nx + wrap(gi + 1, nx);
-        eoN[e] = wrap(gj + 1, ny) * nx + gi;
+    const int tid = ty * (kTX / 2) + tx;
+
+    // offset in the plane of the tiles' pair in row r, pair column p (full
+    // modulo: tiles may be wider than the grid)
+    auto pair_at = [&](int r, int p) -> unsigned {
+        const int gi = ((i0 - 2 + 2 * p) % nx + nx) % nx, gj = ((j0 - 1 + r) % ny + ny) % ny;
+        return (unsigned)gj * nx + gi;
+    };
+    // every thread copies (and corrects) its own pair; the halo pairs, the
+    // tiles' outer rows and then the outer columns of the rows between, go to
+    // the low threads (fields) and to the high ones (pressure)
+    constexpr int XF = L::FCH - NT, XP = L::PCH - NT;
+    static_assert(XF <= NT && XP <= NT, "two pairs a thread");
+    const unsigned gcol = pair_at(ty + 1, tx + 1);
+    const int pos = (ty + 1) * L::FP + 2 * tx + 2, posp = (ty + 1) * L::PP + 2 * tx + 2;
+    const bool more_f = tid < XF, more_p = pc != nullptr && tid >= NT - XP;
+    unsigned gfx, gpx;
+    int sfx, spx, cqx;   // cqx: the halo field pair's place in the pressure tile
+    {
+        constexpr int FC = L::FP / 2, PC = L::PP / 2;
+        int r, p, t = more_f ? tid : 0;
+        if (t < 2 * FC) { r = t < FC ? 0 : BY + 1; p = t < FC ? t : t - FC; }
+        else { t -= 2 * FC; r = 1 + t / 2; p = t % 2 ? FC - 1 : 0; }
+        gfx = pair_at(r, p); sfx = r * L::FP + 2 * p; cqx = r * L::PP + 2 * p;
+        t = more_p ? tid - (NT - XP) : 0;
+        if (t < 3 * PC) { r = t < PC ? 0 : (t < 2 * PC ? BY + 1 : BY + 2); p = t % PC; }
+        else { t -= 3 * PC; r = 1 + t / 3; p = t % 3 == 0 ? 0 : PC - 3 + t % 3; }
+        gpx = pair_at(r, p); spx = r * L::PP + 2 * p;
     }
-    auto load_plane = [&](int kk, int slot) {
-        const int kw = wrap(kk, nz);
-        const long po = (long)kw * plane, pu = (long)wrap(kw + 1, nz) * plane;
+    auto copy_fields = [&](int kk) {
+        const unsigned o = (unsigned)wrap(kk, nz) * plane;
+        double* d = sm.pl[kk & 3][0];
 #pragma unroll
-        for (int e = 0; e < EPT; ++e) {
-            const int t = tid + e * NT;
-            if (t < TP) {
-                double v[NF];
+        for (int f = 0; f < NF; ++f) cp_async<16>(d + f * (L::FP * L::FR) + pos, src[f] + (o + gcol));
+        if (more_f) {
 #pragma unroll
-                for (int f = 0; f < NF; ++f) v[f] = __ldg(src[f] + po + eo[e]);
-                if (pc) {
-                    // the previous step's pressure-gradient correction
-                    // (pressure_solver.f90:98-110), applied where the state is read
-                    const double p0 = __ldg(pc + po + eo[e]);
-                    const double pe = __ldg(pc + po + eoE[e]);
-                    const double pn = __ldg(pc + po + eoN[e]);
-                    const double pt = __ldg(pc + pu + eo[e]);
-                    v[0] = v[0] - a.dtp * (pe - p0) * a.rdx;
-                    v[1] = v[1] - a.dtp * (pn - p0) * a.rdy;
-                    v[2] = (a.rigid && wrap(kw + kofs, nzg) == nzg - 1) ? 0.0 : v[2] - a.dtwp * (pt - p0) * a.rdz;
-                }
-#pragma unroll
-                for (int f = 0; f < NF; ++f) sm.pl[f][slot][t] = v[f];
-            }
+            for (int f = 0; f < NF; ++f) cp_async<16>(d + f * (L::FP * L::FR) + sfx, src[f] + (o + gfx));
+        }
+    };
+    auto copy_p = [&](int kk) {
+        if (!pc) return;
+        const unsigned o = (unsigned)wrap(kk, nz) * plane;
+        double* d = sm.pp[kk & 3];
+        cp_async<16>(d + posp, pc + (o + gcol));
+        if (more_p) cp_async<16>(d + spx, pc + (o + gpx));
+    };
+    // the previous step's pressure-gradient correction
+    // (pressure_solver.f90:98-110) of a landed plane, in place
+    auto correct_pair = [&](int kk, int fpos, int ppos, bool lid) {
+        const double* q = &sm.pp[kk & 3][ppos];
+        const double2 p0 = *reinterpret_cast<const double2*>(q);
+        const double pe = q[2];
+        const double2 pn = *reinterpret_cast<const double2*>(q + L::PP);
+        const double2 pt = *reinterpret_cast<const double2*>(&sm.pp[(kk + 1) & 3][ppos]);
+        constexpr int FS = L::FP * L::FR;
+        double2* u = reinterpret_cast<double2*>(&sm.pl[kk & 3][0][fpos]);
+        double2* v = u + FS / 2;
+        double2* w = v + FS / 2;
+        double2 x = *u, y = *v, z = *w;
+        x.x = x.x - a.dtp * (p0.y - p0.x) * a.rdx;
+        x.y = x.y - a.dtp * (pe - p0.y) * a.rdx;
+        y.x = y.x - a.dtp * (pn.x - p0.x) * a.rdy;
+        y.y = y.y - a.dtp * (pn.y - p0.y) * a.rdy;
+        z.x = lid ? 0.0 : z.x - a.dtwp * (pt.x - p0.x) * a.rdz;
+        z.y = lid ? 0.0 : z.y - a.dtwp * (pt.y - p0.y) * a.rdz;
+        *u = x; *v = y; *w = z;
+    };
+    auto correct = [&](int kk, bool lid) {
+        if (!pc) return;
+        correct_pair(kk, pos, posp, lid);
+        if (more_f) correct_pair(kk, sfx, cqx, lid);
+    };
+    auto is_lid = [&](int kk) { return a.rigid && wrap(wrap(kk, nz) + kofs, nzg) == nzg - 1; };
+    // field f at the thread's pair (or one point) shifted by (di, dj) in a ring slot
+    auto at2 = [&](int s, int f, int dj, double* o) {
+        const double2 v = *reinterpret_cast<const double2*>(&sm.pl[s][f][pos + dj * L::FP]);
+        o[0] = v.x; o[1] = v.y;
+    };
+    auto at1 = [&](int s, int f, int di, int dj) -> double { return sm.pl[s][f][pos + dj * L::FP + di]; };
+
+    // the level's Adams-Bashforth history, into the thread's own slot
+    const bool h1 = a.do_ab && a.ab1 != 0.0, h2 = a.do_ab && a.ab2 != 0.0;
+    auto copy_history = [&](int kk) {
+        const long g = (long)(unsigned)((unsigned)kk * plane + gcol) + ioff;
+        if (h1) {
+            cp_async<sizeof(T2)>(&sm.hist[0][0][tid], (const TT*)a.t1[0] + g);
+            cp_async<sizeof(T2)>(&sm.hist[0][1][tid], (const TT*)a.t1[1] + g);
+            cp_async<sizeof(T2)>(&sm.hist[0][2][tid], (const TT*)a.t1[3] + g);
+            cp_async<16>(&sm.hw[0][tid], (const TW*)a.t1[2] + g);
+        }
+        if (h2) {
+            cp_async<sizeof(T2)>(&sm.hist[1][0][tid], (const TT*)a.t2[0] + g);
+            cp_async<sizeof(T2)>(&sm.hist[1][1][tid], (const TT*)a.t2[1] + g);
+            cp_async<sizeof(T2)>(&sm.hist[1][2][tid], (const TT*)a.t2[3] + g);
+            cp_async<16>(&sm.hw[1][tid], (const TW*)a.t2[2] + g);
         }
     };
 
-    load_plane(kb - 1, (kb + 2) % 3);
-    load_plane(kb, kb % 3);
-    const bool h1 = a.do_ab && a.ab1 != 0.0, h2 = a.do_ab && a.ab2 != 0.0;
-    for (int k = kb; k < ke; ++k) {
-        // history loads first, so they are in flight with the plane's
-        TT hu1 = 0, hv1 = 0, hb1 = 0, hu2 = 0, hv2 = 0, hb2 = 0;
-        double hw1 = 0.0, hw2 = 0.0;
-        const long gh = (long)k * plane + (long)j * nx + i + ioff;
-        if (active && h1) {
-            const TT* const* h = (const TT* const*)a.t1;
-            hu1 = h[0][gh]; hv1 = h[1][gh]; hw1 = ((const TW*)a.t1[2])[gh]; hb1 = h[3][gh];
+    for (int kk = kb - 1; kk <= min(kb + 2, ke); ++kk) copy_fields(kk);
+    for (int kk = kb - 1; kk <= min(kb + 2, ke + 1); ++kk) copy_p(kk);
+    cp_commit();
+    copy_history(kb);
+    cp_commit();
+    cp_wait<1>();
+    __syncthreads();
+    correct(kb - 1, is_lid(kb - 1));
+    __syncthreads();
+    if (kb + 2 <= ke) copy_p(kb + 3);   // into level kb-1's place
+    cp_commit();
+    correct(kb, is_lid(kb));
+    correct(kb + 1, is_lid(kb + 1));
+    cp_wait<0>();
+    __syncthreads();   // three levels corrected; p of level kb+3 has landed
+    const double Ro = a.Ro, rdx = a.rdx, rdy = a.rdy, rdz = a.rdz;
+    const bool rigid = a.rigid;
+    StepCarry c;
+    {
+        const int s2 = (kb - 1) & 3, s0 = kb & 3;
+        const bool bot = rigid && (kb + kofs == 0);   // flux_top(0) = 0
+        double um[2], vm[2], bm[2], wn[2], we[2];
+        at2(s2, 0, 0, um); at2(s2, 1, 0, vm); at2(s2, 2, 0, c.wm); at2(s2, 3, 0, bm);
+        at2(s0, 0, 0, c.u0); at2(s0, 1, 0, c.v0); at2(s0, 2, 0, c.w0); at2(s0, 3, 0, c.b0);
+        c.uw = at1(s0, 0, -1, 0);
+        at2(s0, 1, -1, c.vs);
+        at2(s2, 2, 1, wn);
+        we[0] = c.wm[1]; we[1] = at1(s2, 2, 2, 0);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            c.tb[q] = bot ? 0.0 : (bm[q] + c.b0[q]) * c.wm[q];
+            c.tu[q] = bot ? 0.0 : (c.u0[q] + um[q]) * (c.wm[q] + we[q]);
+            c.tv[q] = bot ? 0.0 : (c.v0[q] + vm[q]) * (c.wm[q] + wn[q]);
+            // rigid lid zeroes flux_top(nz-1:nz+2) for w (advection.f90:167-170)
+            c.tw[q] = (bot || (rigid && kb + kofs >= nzg - 1)) ? 0.0 : (c.w0[q] + c.wm[q]) * (c.wm[q] + c.w0[q]);
+            if constexpr (HARM > 0) {
+                c.hu[q] = bot ? 0.0 : a.Av * (c.u0[q] - um[q]) * rdz;
+                c.hv[q] = bot ? 0.0 : a.Av * (c.v0[q] - vm[q]) * rdz;
+                c.hw[q] = bot ? 0.0 : a.Av * (c.w0[q] - c.wm[q]) * rdz;
+            }
+            if constexpr (HARM > 1) c.hb[q] = bot ? 0.0 : a.Kv * (c.b0[q] - bm[q]) * rdz;
         }
-        if (active && h2) {
-            const TT* const* h = (const TT* const*)a.t2;
-            hu2 = h[0][gh]; hv2 = h[1][gh]; hw2 = ((const TW*)a.t2[2])[gh]; hb2 = h[3][gh];
+        if constexpr (BG) {
+            double U0[2], Um[2], B0[2], Bm[2];
+            at2(s0, 4, 0, U0); at2(s2, 4, 0, Um); at2(s0, 5, 0, B0); at2(s2, 5, 0, Bm);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                c.gu[q] = bot ? 0.0 : 0.25 * (U0[q] + Um[q]) * (c.wm[q] + we[q]);
+                c.gb[q] = bot ? 0.0 : 0.5 * (Bm[q] + B0[q]) * c.wm[q];
+            }
         }
-        load_plane(k + 1, (k + 1) % 3);
-        sm.hu[0][tid] = hu1; sm.hv[0][tid] = hv1; sm.hw[0][tid] = hw1; sm.hb[0][tid] = hb1;
-        sm.hu[1][tid] = hu2; sm.hv[1][tid] = hv2; sm.hw[1][tid] = hw2; sm.hb[1][tid] = hb2;
-        __syncthreads();
-        if (active) {
-            const int sm1 = (k + 2) % 3, s0 = k % 3, sp1 = (k + 1) % 3;
-            auto F = [&](int f, int di, int dj, int dk) -> double {
-                return SM(f, dk < 0 ? sm1 : (dk > 0 ? sp1 : s0), dj, di);
-            };
-            auto Hh = [&](int f, int l) -> double {
-                return f == 0 ? (double)sm.hu[l][tid] : f == 1 ? (double)sm.hv[l][tid]
-                     : f == 2 ? sm.hw[l][tid] : (double)sm.hb[l][tid];
-            };
-            step_point<TT, HARM, WM, BG>(a, F, Hh, i, j, k, ioff, h1, h2);
-        }
-        __syncthreads();
     }
+    __syncthreads();   // level kb-1 is read: its place is filled next
+    // one level; LID: the level may touch the rigid lid
+    auto level = [&](int k, auto lid_c) {
+        constexpr bool LID = decltype(lid_c)::value;
+        const int s0 = k & 3, s1 = (k + 1) & 3;
+        const long g = (long)(unsigned)((unsigned)k * plane + gcol) + ioff;
+        if (k + 3 <= ke) {
+            copy_fields(k + 3);
+            copy_p(k + 4);
+        }
+        cp_commit();
+        [[maybe_unused]] double2 fr[4], fi[4];   // the wavemaker's fields
+        if constexpr (WM) {
+            const unsigned gi = (unsigned)k * plane + gcol;   // within the instance
+#pragma unroll
+            for (int f = 0; f < 4; ++f) {
+                fr[f] = a.wr[f] ? __ldg(reinterpret_cast<const double2*>(a.wr[f] + gi)) : make_double2(0.0, 0.0);
+                fi[f] = a.wi[f] ? __ldg(reinterpret_cast<const double2*>(a.wi[f] + gi)) : make_double2(0.0, 0.0);
+            }
+        }
+        const int kg = k + kofs;                     // global level
+        const bool top = LID && rigid && (kg == nzg - 1);   // flux_top(nz) = 0
+        // rows: [0] is the point west of the pair (U, V, W, B and Un, Ut) or the pair's first (others)
+        double U[4], V[4], W[4], B[4], Us[2], Un[3], Vs[3], Vn[2], Ws[2], Wn[2], Bs[2], Bn[2];
+        double Ut[3], Vt[2], Wt[2], Bt[2], Vst[2];
+        U[0] = c.uw; U[1] = c.u0[0]; U[2] = c.u0[1]; U[3] = at1(s0, 0, 2, 0);
+        V[0] = at1(s0, 1, -1, 0); V[1] = c.v0[0]; V[2] = c.v0[1]; V[3] = at1(s0, 1, 2, 0);
+        W[0] = at1(s0, 2, -1, 0); W[1] = c.w0[0]; W[2] = c.w0[1]; W[3] = at1(s0, 2, 2, 0);
+        B[0] = at1(s0, 3, -1, 0); B[1] = c.b0[0]; B[2] = c.b0[1]; B[3] = at1(s0, 3, 2, 0);
+        at2(s0, 0, -1, Us); Un[0] = at1(s0, 0, -1, 1); at2(s0, 0, 1, Un + 1);
+        Vs[0] = c.vs[0]; Vs[1] = c.vs[1]; Vs[2] = at1(s0, 1, 2, -1); at2(s0, 1, 1, Vn);
+        at2(s0, 2, -1, Ws); at2(s0, 2, 1, Wn);
+        at2(s0, 3, -1, Bs); at2(s0, 3, 1, Bn);
+        Ut[0] = at1(s1, 0, -1, 0); at2(s1, 0, 0, Ut + 1);
+        at2(s1, 1, 0, Vt); at2(s1, 1, -1, Vst); at2(s1, 2, 0, Wt); at2(s1, 3, 0, Bt);
+        double du[2], dv[2], dw[2], db[2], u1[2], v1[2], w1[2], b1[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const double u0 = U[q + 1], v0 = V[q + 1], w0 = W[q + 1], b0 = B[q + 1];
+            const double ue = U[q + 2], uw = U[q], ve = V[q + 2], vw = V[q], we = W[q + 2], ww = W[q];
+            // ---- buoyancy advection + N^2 (advection.f90:12-47, integrate.f90:21-23)
+            // The reference's 0.5 and 0.25 flux factors are powers of two: they
+            // are carried in the per-axis factors a.hd* = 0.5/d*, a.qd* = 0.25/d*
+            // (and 0.25 f0, 0.5 N0^2, set by the launcher), a multiply saved per
+            // flux; scaling by a power of two rounds exactly.  Which of a
+            // difference's two fluxes is rounded before the subtraction is
+            // written out (a point shares fluxes with its pair and with the
+            // level above), so that every form of the kernel gives the same bits.
+            if (a.nonlinear) {
+                {
+                    const double x = __dsub_rn(__dmul_rn(b0 + B[q + 2], u0), __dmul_rn(B[q] + b0, uw));
+                    const double y = __fma_rn(-(Bs[q] + b0), Vs[q], __dmul_rn(b0 + Bn[q], v0));
+                    const double t = top ? 0.0 : __dmul_rn(b0 + Bt[q], w0);
+                    db[q] = -Ro * (x * a.hdx + y * a.hdy + __dsub_rn(t, c.tb[q]) * a.hdz);
+                    c.tb[q] = t;
+                }
+                // ---- zonal momentum (advection.f90:65-100)
+                const double uv = __dmul_rn(u0 + Un[q + 1], ve + v0);          // (u_n)(v_e), also v's eastern flux
+                const double uw_ = __dmul_rn(Ut[q + 1] + u0, w0 + we);         // (u_t)(w_e), also w's eastern flux
+                {
+                    const double x = __fma_rn(u0 + ue, ue + u0, -__dmul_rn(uw + u0, u0 + uw));
+                    const double y = __fma_rn(-(Us[q] + u0), Vs[q + 1] + Vs[q], uv);
+                    const double t = top ? 0.0 : uw_;
+                    du[q] = -Ro * (x * a.qdx + y * a.qdy + __dsub_rn(t, c.tu[q]) * a.qdz);
+                    c.tu[q] = t;
+                }
+                // ---- meridional momentum (advection.f90:104-140)
+                const double vw_ = __dmul_rn(Vt[q] + v0, w0 + Wn[q]);          // (v_t)(w_n), also w's northern flux
+                {
+                    const double x = __fma_rn(-(vw + v0), Un[q] + uw, uv);
+                    const double y = __fma_rn(v0 + Vn[q], Vn[q] + v0, -__dmul_rn(Vs[q] + v0, v0 + Vs[q]));
+                    const double t = top ? 0.0 : vw_;
+                    dv[q] = -Ro * (x * a.qdx + y * a.qdy + __dsub_rn(t, c.tv[q]) * a.qdz);
+                    c.tv[q] = t;
+                }
+                // ---- vertical momentum (advection.f90:145-181)
+                {
+                    const bool wtop = LID && rigid && (kg >= nzg - 2);
+                    const double x = __dsub_rn(uw_, __dmul_rn(ww + w0, uw + Ut[q]));
+                    const double y = __dsub_rn(vw_, __dmul_rn(Ws[q] + w0, Vs[q] + Vst[q]));
+                    const double t = wtop ? 0.0 : __dmul_rn(Wt[q] + w0, w0 + Wt[q]);
+                    dw[q] = -a.dsqr * Ro * (x * a.qdx + y * a.qdy + __dsub_rn(t, c.tw[q]) * a.qdz);
+                    c.tw[q] = t;
+                }
+            } else {
+                db[q] = du[q] = dv[q] = dw[q] = 0.0;
+            }
+            db[q] = db[q] - (w0 + c.wm[q]) * a.hN0sq;
+            // ---- Coriolis, buoyancy force, rigid-lid mask (integrate.f90:37-54)
+            du[q] = du[q] + (v0 + Vs[q] + ve + Vs[q + 1]) * a.qf0;
+            dv[q] = dv[q] - (uw + u0 + Un[q] + Un[q + 1]) * a.qf0;
+            dw[q] = dw[q] + 0.5 * (b0 + Bt[q]);
+            if (top) dw[q] = 0.0;
+            // ---- friction, in place before AB (integrate.f90:59-66)
+            u1[q] = u0; v1[q] = v0; w1[q] = w0; b1[q] = b0;
+            if constexpr (HARM > 0) {
+                const double dt = a.dt;
+#define HARMONIC(f0, fe, fw, fn, fs, ft, Hm, Vm, low, out)                                     \
+    {                                                                                        \
+        const double x = __fma_rn(Hm * (fe - f0), rdx, -__dmul_rn(Hm * (f0 - fw), rdx));     \
+        const double y = __fma_rn(Hm * (fn - f0), rdy, -__dmul_rn(Hm * (f0 - fs), rdy));     \
+        const double t = top ? 0.0 : Vm * (ft - f0) * rdz;                                   \
+        out = f0 + dt * (x * rdx + y * rdy + __dsub_rn(t, low) * rdz);                       \
+        low = t;                                                                             \
+    }
+                if (HARM == 1 || a.harm_uvw) {
+                    HARMONIC(u0, ue, uw, Un[q + 1], Us[q], Ut[q + 1], a.Ah, a.Av, c.hu[q], u1[q])
+                    HARMONIC(v0, ve, vw, Vn[q], Vs[q], Vt[q], a.Ah, a.Av, c.hv[q], v1[q])
+                    HARMONIC(w0, we, ww, Wn[q], Ws[q], Wt[q], a.Ah, a.Av, c.hw[q], w1[q])
+                    if (top) w1[q] = 0.0;
+                }
+                if (HARM > 1 && a.harm_b) HARMONIC(b0, B[q + 2], B[q], Bn[q], Bs[q], Bt[q], a.Kh, a.Kv, c.hb[q], b1[q])
+#undef HARMONIC
+            }
+        }
+        // ---- set_forcing: background-flow advection (lee_wave1.f90:245-312)
+        if constexpr (BG) {
+            double P[4], Pn[3], Ps[2], Pt[3], Q[4], Qn[2], Qs[2], Qt[2];   // U_back, B_back
+            P[0] = at1(s0, 4, -1, 0); at2(s0, 4, 0, P + 1); P[3] = at1(s0, 4, 2, 0);
+            Pn[0] = at1(s0, 4, -1, 1); at2(s0, 4, 1, Pn + 1); at2(s0, 4, -1, Ps);
+            Pt[0] = at1(s1, 4, -1, 0); at2(s1, 4, 0, Pt + 1);
+            Q[0] = at1(s0, 5, -1, 0); at2(s0, 5, 0, Q + 1); Q[3] = at1(s0, 5, 2, 0);
+            at2(s0, 5, 1, Qn); at2(s0, 5, -1, Qs); at2(s1, 5, 0, Qt);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const double u0 = U[q + 1], v0 = V[q + 1], w0 = W[q + 1], b0 = B[q + 1];
+                {
+                    const double x = __fma_rn(-(0.5 * (P[q] + P[q + 1])), u0 + U[q], __dmul_rn(0.5 * (P[q + 1] + P[q + 2]), U[q + 2] + u0));
+                    const double y = __fma_rn(0.25 * (P[q + 1] + Pn[q + 1]), V[q + 2] + v0, -__dmul_rn(0.25 * (Ps[q] + P[q + 1]), Vs[q + 1] + Vs[q]));
+                    const double t = top ? 0.0 : __dmul_rn(0.25 * (Pt[q + 1] + P[q + 1]), w0 + W[q + 2]);
+                    du[q] = du[q] - Ro * (x * rdx + y * rdy + __dsub_rn(t, c.gu[q]) * rdz);
+                    c.gu[q] = t;
+                }
+                {
+                    const double x = __fma_rn(0.25 * (v0 + V[q + 2]), Pn[q + 1] + P[q + 1], -__dmul_rn(0.25 * (V[q] + v0), Pn[q] + P[q]));
+                    dv[q] = dv[q] - Ro * x * rdx;
+                }
+                {
+                    const double x = __fma_rn(0.25 * (w0 + W[q + 2]), P[q + 1] + Pt[q + 1], -__dmul_rn(0.25 * (W[q] + w0), P[q] + Pt[q]));
+                    dw[q] = dw[q] - a.dsqr * Ro * x * rdx;
+                }
+                {
+                    const double e = __fma_rn(0.5 * (b0 + B[q + 2]), P[q + 1], __dmul_rn(0.5 * (Q[q + 1] + Q[q + 2]), u0));
+                    const double em = __fma_rn(0.5 * (B[q] + b0), P[q], __dmul_rn(0.5 * (Q[q] + Q[q + 1]), U[q]));
+                    const double y = __dsub_rn(__dmul_rn(0.5 * (Q[q + 1] + Qn[q]), v0), __dmul_rn(0.5 * (Qs[q] + Q[q + 1]), Vs[q]));
+                    const double t = top ? 0.0 : __dmul_rn(0.5 * (Q[q + 1] + Qt[q]), w0);
+                    db[q] = db[q] - Ro * (__dsub_rn(e, em) * rdx + y * rdy + __dsub_rn(t, c.gb[q]) * rdz);
+                    c.gb[q] = t;
+                }
+            }
+        }
+        // ---- set_forcing: wavemaker (config.f90:224-237)
+        if constexpr (WM) {
+            const double dt = a.dt, cw = a.wm_c, sw = a.wm_s;
+            double* o[4] = {u1, v1, w1, b1};
+#pragma unroll
+            for (int f = 0; f < 4; ++f)
+                if (a.wr[f] || a.wi[f]) {
+                    o[f][0] = o[f][0] + dt * (cw * fr[f].x + sw * fi[f].x);
+                    o[f][1] = o[f][1] + dt * (cw * fr[f].y + sw * fi[f].y);
+                }
+        }
+        // ---- store tendency of time level tau
+        if (active) {
+            T2 t;
+            t.x = (TT)du[0]; t.y = (TT)du[1]; *reinterpret_cast<T2*>((TT*)a.t0[0] + g) = t;
+            t.x = (TT)dv[0]; t.y = (TT)dv[1]; *reinterpret_cast<T2*>((TT*)a.t0[1] + g) = t;
+            *reinterpret_cast<double2*>((TW*)a.t0[2] + g) = make_double2(dw[0], dw[1]);
+            t.x = (TT)db[0]; t.y = (TT)db[1]; *reinterpret_cast<T2*>((TT*)a.t0[3] + g) = t;
+        }
+        // ---- Adams-Bashforth (integrate.f90:87-102)
+        if (a.do_ab) {
+            const double dt = a.dt, dtw = a.dtw;
+            const double c0 = a.ab0, c1 = a.ab1, c2 = a.ab2;
+            // the current tendency enters at full precision; only the
+            // stored history (FP32 in the mixed path) is rounded
+            double tu[2], tv[2], tw[2], tb[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) { tu[q] = c0 * du[q]; tv[q] = c0 * dv[q]; tw[q] = c0 * dw[q]; tb[q] = c0 * db[q]; }
+            cp_wait<1>();   // this level's history has landed (the thread's own copies)
+            auto add = [&](double cc, int l) {
+                const T2 hu = sm.hist[l][0][tid], hv = sm.hist[l][1][tid], hb = sm.hist[l][2][tid];
+                const double2 hw = sm.hw[l][tid];
+                tu[0] = tu[0] + cc * (double)hu.x; tu[1] = tu[1] + cc * (double)hu.y;
+                tv[0] = tv[0] + cc * (double)hv.x; tv[1] = tv[1] + cc * (double)hv.y;
+                tw[0] = tw[0] + cc * hw.x; tw[1] = tw[1] + cc * hw.y;
+                tb[0] = tb[0] + cc * (double)hb.x; tb[1] = tb[1] + cc * (double)hb.y;
+            };
+            if (h1) add(c1, 0);
+            if (h2) add(c2, 1);
+            if (k + 1 < ke) copy_history(k + 1);
+            cp_commit();
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                u1[q] = u1[q] + dt * tu[q]; v1[q] = v1[q] + dt * tv[q];
+                w1[q] = w1[q] + dtw * tw[q]; b1[q] = b1[q] + dt * tb[q];
+            }
+        }
+        if (active) {
+            *reinterpret_cast<double2*>(a.uo + g) = make_double2(u1[0], u1[1]);
+            *reinterpret_cast<double2*>(a.vo + g) = make_double2(v1[0], v1[1]);
+            *reinterpret_cast<double2*>(a.wo + g) = make_double2(w1[0], w1[1]);
+            *reinterpret_cast<double2*>(a.bo + g) = make_double2(b1[0], b1[1]);
+        }
+        c.uw = Ut[0];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            c.wm[q] = W[q + 1];
+            c.u0[q] = Ut[q + 1]; c.v0[q] = Vt[q]; c.w0[q] = Wt[q]; c.b0[q] = Bt[q]; c.vs[q] = Vst[q];
+        }
+        if (k + 2 <= ke) correct(k + 2, LID && is_lid(k + 2));
+        if (a.do_ab) cp_wait<1>();   // the planes; the next level's history may be on its way
+        else cp_wait<0>();
+        __syncthreads();
+    };
+    // levels whose planes stay below the lid go in pairs (the carried values
+    // change registers by name instead of by moves), the others one by one
+    const int km = rigid ? min(ke, nzg - 3 - kofs) : ke;
+    int k = kb;
+#pragma unroll 1
+    for (; k + 1 < km; k += 2) {
+        level(k, std::false_type());
+        level(k + 1, std::false_type());
+    }
+#pragma unroll 1
+    for (; k < ke; ++k) level(k, std::true_type());
 }
 
-template <typename TT, int BY, bool HARM, bool WM, bool BG>
-__global__ void __launch_bounds__(kTX* BY) k_step(const StepArgs a, int kchunk) {
+// Blocks an SM the step kernels are built for: the plain and the u, v, w
+// friction forms fit 168 registers without a spill and run three (247 us FP64,
+// 224-234 us mixed at 256x256x128; held to two 270 and 254 us), the others
+// would spill and run two.
+constexpr int step_blocks(int harm, bool wm, bool bg) { return harm > 1 || wm || bg ? 2 : 3; }
+
+template <typename TT, int BY, int HARM, bool WM, bool BG>
+__global__ void __launch_bounds__(kTX / 2 * BY, step_blocks(HARM, WM, BG)) k_step(const StepArgs a, int kchunk) {
     pdl_trigger();
     pdl_wait();   // the state, p and history were written by the preceding kernels
     step_tile<TT, BY, HARM, WM, BG>(a, kchunk, blockIdx.x, blockIdx.y, blockIdx.z);
@@ -329,8 +504,8 @@ __global__ void __launch_bounds__(kTX* BY) k_step(const StepArgs a, int kchunk) 
 // uneven sizes): block b belongs to the group g with blk0[g] <= b <
 // blk0[g+1] and runs that group's tile as k_step would.  The table rides in
 // the kernel's parameter space (captured by value into a CUDA graph).
-template <typename TT, int BY, bool HARM, bool WM, bool BG>
-__global__ void __launch_bounds__(kTX* BY, BG ? 2 : 4) k_step_groups(const __grid_constant__ StepGroups m) {
+template <typename TT, int BY, int HARM, bool WM, bool BG>
+__global__ void __launch_bounds__(kTX / 2 * BY, step_blocks(HARM, WM, BG)) k_step_groups(const __grid_constant__ StepGroups m) {
     pdl_trigger();
     pdl_wait();
     int g = 0;
@@ -518,18 +693,19 @@ static dim3 prep_step(StepArgs& a, int by) {
     a.qf0 = 0.25 * a.f0; a.hN0sq = 0.5 * a.N0sq;
     const int kcnt = a.kcount ? a.kcount : a.nz;
     a.kchunk = a.kchunk > 0 ? std::min(a.kchunk, kcnt) : (kcnt <= 16 ? kcnt : 8);
+    while ((long)((kcnt + a.kchunk - 1) / a.kchunk) * std::max(1, a.batch) > 65535 && a.kchunk < kcnt) ++a.kchunk;   // the grid's z limit
     return dim3((a.nx + kTX - 1) / kTX, (a.ny + by - 1) / by, ((kcnt + a.kchunk - 1) / a.kchunk) * std::max(1, a.batch));
 }
 
-template <typename TT, int BY, bool HARM, bool WM, bool BG>
+template <typename TT, int BY, int HARM, bool WM, bool BG>
 static cudaError_t launch_step_t(const StepArgs& a0, cudaStream_t s) {
     StepArgs a = a0;
     const dim3 grid = prep_step(a, BY);
-    return launch_pdl(k_step<TT, BY, HARM, WM, BG>, grid, dim3(kTX, BY), sizeof(StepSmem<TT, BY, BG ? 6 : 4>), s, a,
+    return launch_pdl(k_step<TT, BY, HARM, WM, BG>, grid, dim3(kTX / 2, BY), sizeof(StepSmem<TT, BY, BG ? 6 : 4>), s, a,
                       a.kchunk);
 }
 
-template <typename TT, int BY, bool HARM, bool WM, bool BG>
+template <typename TT, int BY, int HARM, bool WM, bool BG>
 static cudaError_t launch_step_groups_t(const StepArgs* in, int n, cudaStream_t s) {
     static_assert(sizeof(StepGroups) <= 32000, "grouped step table exceeds the kernel parameter space");
     StepGroups m{};
@@ -544,13 +720,30 @@ static cudaError_t launch_step_groups_t(const StepArgs* in, int n, cudaStream_t 
     }
     if (blocks > 0x7fffffffL) return cudaErrorInvalidValue;
     m.blk0[n] = (int)blocks;
-    return launch_pdl(k_step_groups<TT, BY, HARM, WM, BG>, dim3((unsigned)blocks), dim3(kTX, BY),
+    return launch_pdl(k_step_groups<TT, BY, HARM, WM, BG>, dim3((unsigned)blocks), dim3(kTX / 2, BY),
                       sizeof(StepSmem<TT, BY, BG ? 6 : 4>), s, m);
 }
 
+// friction of u, v, w alone (1) or of b as well (2), wavemaker, background flow
 int step_flavour(const StepArgs& a) {
-    return (a.harm_uvw || a.harm_b ? 1 : 0) | (a.wm_on ? 2 : 0) | (a.ub ? 4 : 0);
+    return (a.harm_b ? 2 : (a.harm_uvw ? 1 : 0)) | (a.wm_on ? 4 : 0) | (a.ub ? 8 : 0);
 }
+// F(harm, wm, bg) for the instantiation that a flavour runs
+#define PS3D_STEP_DISPATCH(flavour, F)                                                            \
+    switch (flavour) {                                                                           \
+        case 0: F(0, false, false); break;                                                       \
+        case 1: F(1, false, false); break;                                                       \
+        case 2: F(2, false, false); break;                                                       \
+        case 4: F(0, true, false); break;                                                        \
+        case 5: F(1, true, false); break;                                                        \
+        case 6: F(2, true, false); break;                                                        \
+        case 8: F(0, false, true); break;                                                        \
+        case 9: F(1, false, true); break;                                                        \
+        case 10: F(2, false, true); break;                                                       \
+        case 12: F(0, true, true); break;                                                        \
+        case 13: F(1, true, true); break;                                                        \
+        default: F(2, true, true); break;                                                        \
+    }
 
 template <typename TT>
 static cudaError_t launch_step_groups_tt(const StepArgs* a, int n, cudaStream_t s) {
@@ -559,17 +752,9 @@ static cudaError_t launch_step_groups_tt(const StepArgs* a, int n, cudaStream_t 
     for (int g = 1; g < n; ++g)
         if (step_flavour(a[g]) != fl) return cudaErrorInvalidValue;
 #define L(H, W, G) return launch_step_groups_t<TT, 8, H, W, G>(a, n, s)
-    switch (fl) {
-        case 0: L(false, false, false);
-        case 1: L(true, false, false);
-        case 2: L(false, true, false);
-        case 3: L(true, true, false);
-        case 4: L(false, false, true);
-        case 5: L(true, false, true);
-        case 6: L(false, true, true);
-        default: L(true, true, true);
-    }
+    PS3D_STEP_DISPATCH(fl, L)
 #undef L
+    return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_step_groups(const StepArgs* a, int n, bool fp32_tendencies, cudaStream_t s) {
@@ -578,13 +763,10 @@ cudaError_t launch_step_groups(const StepArgs* a, int n, bool fp32_tendencies, c
 
 template <typename TT>
 static cudaError_t launch_step_tt(const StepArgs& a, cudaStream_t s) {
-    const bool harm = a.harm_uvw || a.harm_b;
-    const bool wm = a.wm_on != 0;
-    const bool bg = a.ub != nullptr;
 #define L(H, W, G) return launch_step_t<TT, 8, H, W, G>(a, s)
-    if (harm) { if (wm) { if (bg) L(true, true, true); else L(true, true, false); } else { if (bg) L(true, false, true); else L(true, false, false); } }
-    else { if (wm) { if (bg) L(false, true, true); else L(false, true, false); } else { if (bg) L(false, false, true); else L(false, false, false); } }
+    PS3D_STEP_DISPATCH(step_flavour(a), L)
 #undef L
+    return cudaErrorInvalidValue;
 }
 
 template <typename TT>
@@ -606,8 +788,10 @@ static cudaError_t step_setup_tt() {
         (e = cudaFuncSetAttribute(k_step<TT, 8, H, W, G>, cudaFuncAttributePreferredSharedMemoryCarveout,  \
                                   carve)))                                                                \
         return e;
-    S(true, true, true) S(true, true, false) S(true, false, true) S(true, false, false)
-    S(false, true, true) S(false, true, false) S(false, false, true) S(false, false, false)
+    for (int fl = 0; fl < 15; ++fl) {
+        if (fl % 4 == 3) continue;
+        PS3D_STEP_DISPATCH(fl, S)
+    }
 #undef S
     return cudaSuccess;
 }
@@ -624,18 +808,9 @@ static int step_resident_tt(const StepArgs& a) {
     int n = 0;
     cudaError_t e = cudaSuccess;
 #define R(H, W, G)                                                                                            \
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_step<TT, 8, H, W, G>, kTX * 8,                   \
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_step<TT, 8, H, W, G>, kTX / 2 * 8,                   \
                                                       sizeof(StepSmem<TT, 8, G ? 6 : 4>));
-    switch (step_flavour(a)) {
-        case 0: R(false, false, false) break;
-        case 1: R(true, false, false) break;
-        case 2: R(false, true, false) break;
-        case 3: R(true, true, false) break;
-        case 4: R(false, false, true) break;
-        case 5: R(true, false, true) break;
-        case 6: R(false, true, true) break;
-        default: R(true, true, true) break;
-    }
+    PS3D_STEP_DISPATCH(step_flavour(a), R)
 #undef R
     if (e != cudaSuccess) { cudaGetLastError(); return 1; }
     return n > 0 ? n : 1;
