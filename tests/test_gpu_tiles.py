@@ -1,0 +1,87 @@
+"""Edges of the kernels' tiles and batches: grids that are no multiple of a
+tile, the smallest grids, z chunks of every size, against the oracle or
+bit for bit against another split of the same work."""
+import numpy as np
+import pytest
+
+from ps3d_b200 import abi
+from ps3d_b200 import configs as cf
+from ps3d_b200.model import Model
+from oracle.binding import Oracle
+from tests.helpers import FIELDS, compare_state, load_oracle, small_params, smooth_state, upload_from_oracle
+
+pytestmark = pytest.mark.gpu
+TOL64 = 1e-11   # several FP64 steps: the suite's bound for rounding in another order
+
+FRICTION = {"none": dict(Ah=0.0, Av=0.0), "uvw": {}, "uvwb": dict(Kh=2e-2, Kv=1e-2)}
+
+
+def _pair(p, f):
+    o, m = Oracle(p), Model(p)
+    load_oracle(o, f)
+    upload_from_oracle(m, o)
+    return o, m
+
+
+@pytest.mark.parametrize("friction", sorted(FRICTION))
+@pytest.mark.parametrize("n", [(4, 4, 2), (36, 10, 3), (64, 8, 5), (30, 18, 7)])
+@pytest.mark.parametrize("rigid", [True, False])
+def test_step_at_tile_edges(n, friction, rigid):
+    """Four AB3 steps (cold, one and two history levels, a pending
+    correction) on grids narrower and wider than the 32 x 8 column tile."""
+    nz = n[2] if rigid else max(2, 2 * (n[2] // 2))
+    p = small_params(n[0], n[1], nz, rigid=rigid, **FRICTION[friction])
+    o, m = _pair(p, smooth_state(p, seed=31))
+    o.integrate(4)
+    m.run(4)
+    err = compare_state(m, o)
+    assert max(err.values()) < TOL64, err
+
+
+@pytest.mark.parametrize("forced", [False, True])
+@pytest.mark.parametrize("precision", [abi.PS3D_FP64, abi.PS3D_MIXED])
+def test_step_z_chunks_give_the_same_bits(precision, forced, monkeypatch):
+    """Any z chunk of the step kernel (a block's carried fluxes start anew at
+    every chunk) gives the same bits."""
+    ref = None
+    for kc in (13, 1, 2, 3, 5):
+        monkeypatch.setenv("PS3D_TUNE", f"im0,C1,rc4,tj8,ly8,pol1,kc{kc}")
+        p = small_params(36, 20, 13, rigid=True, precision=precision)
+        if forced:
+            p.Ah = p.Av = 0.0
+        m = Model(p)
+        f = smooth_state(p, seed=32)
+        m.upload(**{k: f[k] for k in FIELDS})
+        if forced:
+            rng = np.random.default_rng(33)
+            g = {k: cf.halo_fill(a * rng.standard_normal(m.shape)) for k, a in
+                 (("w_r", 1e-6), ("b_i", 1e-8), ("u_back", 0.1), ("b_back", 1e-4))}
+            m.set_forcing(abi.PS3D_FORCE_WAVEMAKER | abi.PS3D_FORCE_BACKGROUND, omega=5e-4, **g)
+        m.run(5)
+        got = m.download()
+        assert f"kchunk={kc}" in m.describe()
+        if ref is None:
+            ref = got
+        for k in FIELDS + ("p", "du", "dv", "dw", "db"):
+            assert np.array_equal(got[k], ref[k]), (kc, k)
+
+
+@pytest.mark.parametrize("n", [(2, 2, 2), (4, 2, 3), (30, 18, 7), (270, 4, 5)])
+def test_halo_layout_round_trip(n):
+    """Upload takes the interior, download fills the halos periodically (p
+    under a rigid lid: the nearest level), exactly."""
+    p = small_params(*n, rigid=True, precision=abi.PS3D_FP64)
+    m = Model(p)
+    rng = np.random.default_rng(34)
+    up = {k: rng.standard_normal(m.shape) for k in FIELDS + ("p",)}
+    up["du"] = rng.standard_normal((3,) + m.shape)
+    m.upload(**up)
+    got = m.download()
+    for k in FIELDS:
+        assert np.array_equal(got[k], cf.halo_fill(up[k].copy())), k
+    want = cf.halo_fill(up["p"].copy())
+    for z, s in ((0, 2), (1, 2), (-1, -3), (-2, -3)):
+        want[z] = want[s]
+    assert np.array_equal(got["p"], want)
+    for s in range(3):
+        assert np.array_equal(got["du"][s], cf.halo_fill(up["du"][s].copy()))
