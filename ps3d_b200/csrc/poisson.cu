@@ -1033,12 +1033,29 @@ cudaError_t launch_colsolve(const PlaneArgs& p, const ColumnArgs& c, cudaStream_
 // ---------------------------------------------------------------------------
 constexpr int kZLines = 32;
 
+// the spectral value times -1/ksqr (pressure_solver.f90:59-69), zero where
+// ksqr is; FP64 forms one reciprocal for both parts, FP32 divides in FP64
 template <typename R>
-__global__ void __launch_bounds__(256) k_zsolve(const ColumnArgs a) {
+__device__ __forceinline__ cpx<R> z_divide(cpx<R> v, double ks) {
+    if (!(ks > 0.0)) return mk<R>((R)0, (R)0);
+    if constexpr (sizeof(R) == 8) {
+        const double r = -1.0 / ks;
+        return mk<R>(v.x * r, v.y * r);
+    } else {
+        return mk<R>((R)(-(double)v.x / ks), (R)(-(double)v.y / ks));
+    }
+}
+
+// Columns staged in shared memory, any length that factors: a lane keeps one
+// column, so no index is divided (256x256x96 FP64 92 -> 59 us, FP32 90 -> 51).
+template <typename R>
+__global__ void __launch_bounds__(256, 2) k_zsolve(const ColumnArgs a) {
+    pdl_trigger();
+    pdl_wait();   // inputs written by the preceding kernels
     using T = cpx<R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T* buf = reinterpret_cast<T*>(smem_raw);
-    const int ld = kZLines + 1;
+    constexpr int ld = kZLines + 1;
     const int nz = a.nz;
     const PlanTables<R> tz = stage_plan<R>(a.pz, smem_raw + align16((size_t)nz * ld * sizeof(T)));
     const long ncols = a.ncl ? a.ncl : (long)a.nxh * a.ny;   // columns held (a column slab: ncl)
@@ -1046,39 +1063,139 @@ __global__ void __launch_bounds__(256) k_zsolve(const ColumnArgs a) {
     const long inst = blockIdx.x / bpi;
     const long c0 = (blockIdx.x - inst * bpi) * (long)kZLines;
     const int nl = (int)min((long)kZLines, ncols - c0);
-    T* spec = reinterpret_cast<T*>(a.spec) + inst * a.sM;
-    __syncthreads();
-    for (int t = threadIdx.x; t < nz * nl; t += blockDim.x) {
-        const int k = t / nl, l = t - k * nl;
-        const int slot = (a.op == 2) ? tz.pos[k] : k;
-        buf[slot * ld + l] = spec[c0 + l + (long)k * ncols];
+    const int l = threadIdx.x % kZLines, kw = threadIdx.x / kZLines, nw = 256 / kZLines;
+    const unsigned long long pk = pol_keep(a.l2hint);
+    T* spec = reinterpret_cast<T*>(a.spec) + inst * a.sM + c0 + l;
+    const bool on = l < nl;
+    constexpr int LB = sizeof(R) == 8 ? 4 : 8;
+    __syncthreads();   // the tables are staged (op 2 places by them)
+    for (int k0 = kw; k0 < nz; k0 += LB * nw) {
+        T v[LB];
+#pragma unroll
+        for (int q = 0; q < LB; ++q)
+            if (on && k0 + q * nw < nz) v[q] = ld_l2(spec + (long)(k0 + q * nw) * ncols, pk);
+#pragma unroll
+        for (int q = 0; q < LB; ++q) {
+            const int k = k0 + q * nw;
+            if (on && k < nz) buf[((a.op == 2) ? tz.pos[k] : k) * ld + l] = v[q];
+        }
     }
     if (a.op == 2) {
-        fft_batch<true, R>(buf, ld, nl, a.pz, +1, tz.tw);
+        fft_batch<true, R, 16, true>(buf, ld, nl, a.pz, +1, tz.tw, kZLines);
     } else {
-        fft_batch<false, R>(buf, ld, nl, a.pz, -1, tz.tw);
+        fft_batch<false, R, 16, true>(buf, ld, nl, a.pz, -1, tz.tw, kZLines);
         const R sc = (R)a.scale;
-        for (int t = threadIdx.x; t < nz * nl; t += blockDim.x) {
-            const int p = t / nl, l = t - p * nl;
-            T v = cscale(buf[p * ld + l], sc);
-            if (a.op == 0) {
-                const long c = c0 + l + a.col0;   // global column: its wavenumbers
-                const int i = a.layout ? (int)(c / a.ny) : (int)(c % a.nxh);
-                const int j = a.layout ? (int)(c % a.ny) : (int)(c / a.nxh);
-                const int k = tz.ipos[p];
-                const double ks = a.hkx[i] + a.hky[j] + a.hkz[k];
-                if (ks > 0.0) { v.x = (R)(-(double)v.x / ks); v.y = (R)(-(double)v.y / ks); }
-                else { v.x = (R)0; v.y = (R)0; }
-            }
-            buf[p * ld + l] = v;
+        double k2 = 0.0;
+        if (a.op == 0 && on) {
+            const long c = c0 + l + a.col0;   // global column: its wavenumbers
+            k2 = a.hkx[a.layout ? c / a.ny : c % a.nxh] + a.hky[a.layout ? c % a.ny : c / a.nxh];
         }
-        if (a.op == 0) fft_batch<true, R>(buf, ld, nl, a.pz, +1, tz.tw);
+        if (on)
+            for (int p = kw; p < nz; p += nw) {
+                T v = cscale(buf[p * ld + l], sc);
+                if (a.op == 0) v = z_divide<R>(v, k2 + a.hkz[tz.ipos[p]]);
+                buf[p * ld + l] = v;
+            }
+        if (a.op == 0) fft_batch<true, R, 16, true>(buf, ld, nl, a.pz, +1, tz.tw, kZLines);
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < nz * nl; t += blockDim.x) {
-        const int k = t / nl, l = t - k * nl;
-        const int slot = (a.op == 1) ? tz.pos[k] : k;
-        spec[c0 + l + (long)k * ncols] = buf[slot * ld + l];
+    if (on)
+        for (int k = kw; k < nz; k += nw) st_l2(spec + (long)k * ncols, buf[((a.op == 1) ? tz.pos[k] : k) * ld + l], pk);
+}
+
+// The same with the columns in registers, for nz = 16 N1 (32, 64, 128, 256):
+// the four-step split of the y lines (k_ylines_reg) with the column index
+// across the lanes, so that every level is read and written in runs of CL
+// columns.  A column is N1 threads of 16 elements each.
+//   forward  thread t takes n2 = t, t + N1, ..: DFT N1 over x[16 n1 + n2],
+//            w_nz^(n2 k1), through shared memory to thread k1, DFT 16;
+//   divide   thread k1 holds X[k1 + N1 k2] for every k2;
+//   inverse  the same steps backwards, ending on the elements it loaded.
+// Two shared-memory round trips an element against the staged kernel's six
+// (bound by them and by its latency at three blocks an SM).  The butterflies
+// and twiddles are the staged kernel's for the plan {16, N1}, in its order:
+// the same bits in FP32 (in FP64 too but for the shared reciprocal).
+// Bound by its FP64 arithmetic and two block barriers at four blocks an SM:
+// 512x256x128 80 us FP64 (270 MB, 52 % of the copy bandwidth) and 64 us FP32,
+// where the staged kernel with divided indices took 206 and 165 us.
+constexpr int kZRegThreads = 128;
+
+template <typename R, int N1>
+__global__ void __launch_bounds__(kZRegThreads, 4) k_zsolve_reg(const ColumnArgs a) {
+    pdl_trigger();
+    pdl_wait();   // inputs written by the preceding kernels
+    using T = cpx<R>;
+    constexpr int N2 = 16, CL = kZRegThreads / N1, NS = N2 / N1;
+    __shared__ __align__(16) unsigned char z_raw[kZRegThreads * 16 * sizeof(T)];
+    T* buf = reinterpret_cast<T*>(z_raw);   // [k1][n2][column]
+    const int l = threadIdx.x % CL, t = threadIdx.x / CL;
+    const long ncols = a.ncl ? a.ncl : (long)a.nxh * a.ny;
+    const long bpi = (ncols + CL - 1) / CL;
+    const long inst = blockIdx.x / bpi;
+    const long c0 = (blockIdx.x - inst * bpi) * (long)CL + l;
+    const bool on = c0 < ncols;
+    const unsigned long long pk = pol_keep(a.l2hint);
+    T* spec = reinterpret_cast<T*>(a.spec) + inst * a.sM + (on ? c0 : 0);
+    const T* tw = reinterpret_cast<const T*>(sizeof(R) == 8 ? (const void*)a.pz.tw : (const void*)a.pz.twf);
+    T v[16];
+    if (a.op != 2) {
+#pragma unroll
+        for (int s = 0; s < NS; ++s)
+#pragma unroll
+            for (int n1 = 0; n1 < N1; ++n1) v[s * N1 + n1] = ld_l2(spec + (long)(N2 * n1 + t + N1 * s) * ncols, pk);
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            const int n2 = t + N1 * s;
+            small_dft<N1>(v + s * N1, -1);
+#pragma unroll
+            for (int k1 = 1; k1 < N1; ++k1)
+                if (n2) v[s * N1 + k1] = cmul(v[s * N1 + k1], __ldg(tw + n2 * k1));
+#pragma unroll
+            for (int k1 = 0; k1 < N1; ++k1) buf[(k1 * N2 + n2) * CL + l] = v[s * N1 + k1];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int n2 = 0; n2 < N2; ++n2) v[n2] = buf[(t * N2 + n2) * CL + l];
+        small_dft<N2>(v, -1);   // v[k2] = X[t + N1 k2]
+        const R sc = (R)a.scale;
+        if (a.op == 0) {
+            const long c = (on ? c0 : 0) + a.col0;   // global column: its wavenumbers
+            const double k2s = a.hkx[a.layout ? c / a.ny : c % a.nxh] + a.hky[a.layout ? c % a.ny : c / a.nxh];
+#pragma unroll
+            for (int k2 = 0; k2 < N2; ++k2) v[k2] = z_divide<R>(cscale(v[k2], sc), k2s + __ldg(a.hkz + t + N1 * k2));
+        } else {
+            if (on) {
+#pragma unroll
+                for (int k2 = 0; k2 < N2; ++k2) st_l2(spec + (long)(t + N1 * k2) * ncols, cscale(v[k2], sc), pk);
+            }
+            return;
+        }
+    } else {
+#pragma unroll
+        for (int k2 = 0; k2 < N2; ++k2) v[k2] = ld_l2(spec + (long)(t + N1 * k2) * ncols, pk);
+    }
+    small_dft<N2>(v, +1);
+#pragma unroll
+    for (int n2 = 0; n2 < N2; ++n2) buf[(t * N2 + n2) * CL + l] = v[n2];   // the slots this thread read
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        const int n2 = t + N1 * s;
+#pragma unroll
+        for (int k1 = 0; k1 < N1; ++k1) {
+            T x = buf[(k1 * N2 + n2) * CL + l];
+            if (k1 && n2) {
+                T w = __ldg(tw + n2 * k1);
+                w.y = -w.y;
+                x = cmul(x, w);
+            }
+            v[s * N1 + k1] = x;
+        }
+        small_dft<N1>(v + s * N1, +1);
+        if (on) {
+#pragma unroll
+            for (int n1 = 0; n1 < N1; ++n1) st_l2(spec + (long)(N2 * n1 + n2) * ncols, v[s * N1 + n1], pk);
+        }
     }
 }
 
@@ -2075,15 +2192,37 @@ bool zsolve_fits(int nz, bool fp32) {
     return zsolve_smem(nz, fp32 ? sizeof(float2) : sizeof(double2)) <= 227 * 1024;
 }
 
-cudaError_t launch_zsolve(const ColumnArgs& a, bool fp32, cudaStream_t s) {
+// Columns in registers where the plan's radices are {16, N1}: nz = 32 (9.8 us
+// at 64x66x32x3, staged 13.6), 64 (11.4, 16.0 at 128x64), 128 (80, 206 at
+// 512x256), 256 (11.8, 40.6 at 32x32).  Every other length is staged
+// (PS3D_ZSOLVE=0 stages all).
+template <typename R, int N1>
+static cudaError_t launch_zsolve_reg(const ColumnArgs& a, cudaStream_t s) {
+    const long ncols = a.ncl ? a.ncl : (long)a.nxh * a.ny;
+    constexpr int CL = kZRegThreads / N1;
+    const long blocks = (ncols + CL - 1) / CL * std::max(1, a.batch);
+    return launch_pdl(k_zsolve_reg<R, N1>, dim3((unsigned)blocks), dim3(kZRegThreads), 0, s, a);
+}
+
+cudaError_t launch_zsolve(const ColumnArgs& a0, bool fp32, cudaStream_t s) {
+    ColumnArgs a = a0;
+    a.l2hint = l2hint_mode();
+    const char* pin = std::getenv("PS3D_ZSOLVE");
+    if (a.pz.nst == 2 && a.pz.r[0] == 16 && !(pin && pin[0] == '0')) {
+        switch (a.pz.r[1]) {
+            case 2: return fp32 ? launch_zsolve_reg<float, 2>(a, s) : launch_zsolve_reg<double, 2>(a, s);
+            case 4: return fp32 ? launch_zsolve_reg<float, 4>(a, s) : launch_zsolve_reg<double, 4>(a, s);
+            case 8: return fp32 ? launch_zsolve_reg<float, 8>(a, s) : launch_zsolve_reg<double, 8>(a, s);
+            case 16: return fp32 ? launch_zsolve_reg<float, 16>(a, s) : launch_zsolve_reg<double, 16>(a, s);
+        }
+    }
     const long ncols = a.ncl ? a.ncl : (long)a.nxh * a.ny;
     const int blocks = (int)(((ncols + kZLines - 1) / kZLines) * std::max(1, a.batch));
     const size_t es = fp32 ? sizeof(float2) : sizeof(double2);
     const size_t sm = zsolve_smem(a.nz, es);
     if (sm > 227 * 1024) return cudaErrorInvalidValue;
-    if (fp32) k_zsolve<float><<<blocks, 256, sm, s>>>(a);
-    else k_zsolve<double><<<blocks, 256, sm, s>>>(a);
-    return cudaGetLastError();
+    if (fp32) return launch_pdl(k_zsolve<float>, dim3(blocks), dim3(256), sm, s, a);
+    return launch_pdl(k_zsolve<double>, dim3(blocks), dim3(256), sm, s, a);
 }
 
 }  // namespace ps3d
