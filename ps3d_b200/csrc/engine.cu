@@ -534,11 +534,17 @@ int Ctx::step(int itt_, int tau_, int taum1_, int taum2_) {
     }
     const bool fused = fused_step();
     if (split_solve && !fused) return PS3D_ERR_UNSUPPORTED;   // z-slabs: the fused step only
-    if (!fused) {
+    // biharmonic friction without a callback or a background flow: the step
+    // kernel, then every friction stage, the wavemaker and Adams-Bashforth in
+    // one kernel.  Without harmonic friction the step kernel's output is the
+    // corrected start-of-step state, so the correction can stay pending.
+    const bool bihf = !fused && bih && !cb && !bg;
+    const bool lazy_in = fused || (bihf && !harm);
+    if (!lazy_in) {
         int rc = materialize();
         if (rc) return rc;
     }
-    if (fused && pending) {
+    if (lazy_in && pending) {
         a.pc = pcor;
         a.dtp = dtp;
         a.dtwp = dtp / P.dsqr;
@@ -565,6 +571,26 @@ int Ctx::step(int itt_, int tau_, int taum1_, int taum2_) {
         a.wm_on = 0;
         StepArgs k1 = a;
         LAUNCH(PS3D_K_STEP, launch_step(k1, false, stream));
+        if (bihf) {
+            pending = false;   // consumed by the step kernel
+            FrictionArgs fr{};
+            fr.nx = nx; fr.ny = ny; fr.nz = nz; fr.rigid = rigid;
+            fr.rdx = a.rdx; fr.rdy = a.rdy; fr.rdz = a.rdz; fr.dt = P.dt; fr.dtw = a.dtw;
+            fr.ab0 = a.ab0; fr.ab1 = a.ab1; fr.ab2 = a.ab2;
+            fr.wm_on = wm; fr.wm_c = a.wm_c; fr.wm_s = a.wm_s;
+            for (int f = 0; f < 4; ++f) {
+                fr.hmix[f] = f < 3 ? P.Ahbi : P.Khbi;
+                fr.vmix[f] = f < 3 ? P.Avbi : P.Kvbi;
+                fr.h[f] = (const double*)state[f][B[f]].p;
+                fr.old[f] = harm ? (const double*)state[f][old[f]].p : fr.h[f];
+                fr.out[f] = (double*)state[f][Cb[f]].p;
+                fr.t0[f] = (const double*)a.t0[f]; fr.t1[f] = (const double*)a.t1[f]; fr.t2[f] = (const double*)a.t2[f];
+                fr.wr[f] = a.wr[f]; fr.wi[f] = a.wi[f];
+            }
+            LAUNCH(PS3D_K_OTHER, launch_friction(fr, stream));
+            for (int f = 0; f < 4; ++f) cur[f] = Cb[f];
+            return pressure_solve(lazy_correction);
+        }
         int fin[4] = {B[0], B[1], B[2], B[3]};
         // biharmonic_h then biharmonic_v per field (integrate.f90:68-78)
         const double rdx = a.rdx, rdy = a.rdy, rdz = a.rdz;

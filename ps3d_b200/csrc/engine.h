@@ -78,6 +78,23 @@ struct StepGroups {
     int n;
 };
 
+// Biharmonic friction, wavemaker and Adams-Bashforth in one pass (FP64, one
+// grid), after a step kernel launched with do_ab = 0.
+struct FrictionArgs {
+    int nx, ny, nz, rigid;
+    double rdx, rdy, rdz, dt, dtw;
+    double ab0, ab1, ab2;
+    double hmix[4], vmix[4];       // biharmonic coefficients of u, v, w, b (0: none)
+    const double* h[4];            // the step kernel's output: u, v, w, b after harmonic friction
+    const double* old[4];          // start-of-step fields (read beyond the interior)
+    double* out[4];
+    const double *t0[4], *t1[4], *t2[4];
+    int wm_on;
+    double wm_c, wm_s;
+    const double *wr[4], *wi[4];
+    int kchunk;                    // set by launch_friction
+};
+
 // Plane-FFT kernels (divergence + forward 2D FFT, inverse 2D FFT) for one grid.
 struct PlaneArgs {
     int nx, ny, nz, nxh;
@@ -159,6 +176,7 @@ int step_resident(const StepArgs& a, bool fp32_tendencies);
 // one launch of the step kernel over n <= kMaxStepGroups grids, each as
 // launch_step(a[g], fp32_tendencies) would step it
 cudaError_t launch_step_groups(const StepArgs* a, int n, bool fp32_tendencies, cudaStream_t s);
+cudaError_t launch_friction(const FrictionArgs& a, cudaStream_t s);
 cudaError_t launch_biharmonic_h(const double* cur, const double* old, double* out, int nx, int ny, int nz,
                                 double Hmix, double rdx, double rdy, double dt, cudaStream_t s);
 cudaError_t launch_biharmonic_v(const double* cur, const double* old, double* out, int nx, int ny, int nz,

@@ -577,6 +577,172 @@ __global__ void k_biharmonic_v(const double* __restrict__ cur, const double* __r
     }
 }
 
+// ---------------------------------------------------------------------------
+// Biharmonic friction of all four fields, wavemaker and Adams-Bashforth in one
+// pass over the step kernel's output (mixing.f90:96-217, config.f90:224-237,
+// integrate.f90:68-102), where the stages above are a pass over memory each.
+// A block marches up in z with the planes of the harmonic-updated fields in a
+// three-slot ring (16-byte asynchronous copies, two points of halo); a thread
+// applies the horizontal operator to its pair of points as a plane arrives
+// and keeps the five levels that the vertical operator needs in registers.
+// A neighbour outside the interior is read from the start-of-step field, as
+// the reference's unexchanged halos hold it.
+// 160 B a point (fields and three tendency levels read, fields written);
+// 128x128x64 takes 47 us (3.6 TB/s; two blocks of 240 registers an SM wait on
+// their FP64 chains), where eight friction passes, the wavemaker and
+// Adams-Bashforth pass and the correction pass took 243 us.
+// ---------------------------------------------------------------------------
+template <int BY>
+struct FrictionTile {
+    static constexpr int NT = kTX / 2 * BY;
+    static constexpr int FP = kTX + 4, FR = BY + 4, FS = FP * FR;   // columns i0-2 .. i0+33, rows j0-2 .. j0+BY+1
+    static constexpr int XF = FP / 2 * FR - NT;                     // halo pairs
+};
+
+template <int BY>
+__global__ void __launch_bounds__(kTX / 2 * BY, 2) k_friction_ab(const FrictionArgs a) {
+    using L = FrictionTile<BY>;
+    constexpr int NT = L::NT;
+    static_assert(L::XF <= NT, "one halo pair a thread");
+    pdl_trigger();
+    pdl_wait();   // inputs written by the preceding kernels
+    __shared__ __align__(16) double ring[3][4][L::FS];
+    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * (kTX / 2) + tx;
+    const int nx = a.nx, ny = a.ny, nz = a.nz;
+    const int i0 = blockIdx.x * kTX, j0 = blockIdx.y * BY;
+    const int kb = blockIdx.z * a.kchunk, ke = min(nz, kb + a.kchunk);
+    const bool active = (i0 + 2 * tx < nx) && (j0 + ty < ny);   // threads past the edge run along, storing nothing
+    const unsigned plane = (unsigned)nx * ny;
+    auto pair_at = [&](int r, int p, bool& in) -> unsigned {
+        const int x = i0 - 2 + 2 * p, y = j0 - 2 + r;
+        in = x >= 0 && x < nx && y >= 0 && y < ny;
+        return (unsigned)((y % ny + ny) % ny) * nx + (x % nx + nx) % nx;
+    };
+    bool in0, inx;
+    const unsigned gcol = pair_at(ty + 2, tx + 1, in0);
+    const int pos = (ty + 2) * L::FP + 2 * tx + 2;
+    const bool more = tid < L::XF;
+    unsigned gx;
+    int sx;
+    {
+        constexpr int FC = L::FP / 2;
+        int r, p, t = more ? tid : 0;
+        if (t < 4 * FC) { r = t / FC; p = t - r * FC; r = r < 2 ? r : BY + r; }
+        else { t -= 4 * FC; r = 2 + t / 2; p = t % 2 ? FC - 1 : 0; }
+        gx = pair_at(r, p, inx);
+        sx = r * L::FP + 2 * p;
+    }
+    auto copy_plane = [&](int m) {
+        const bool lin = m >= 0 && m < nz;
+        const unsigned o = (unsigned)wrap(m, nz) * plane;
+        double* d = ring[(m + 3) % 3][0];
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+            cp_async<16>(d + f * L::FS + pos, (lin && in0 ? a.h[f] : a.old[f]) + (o + gcol));
+            if (more) cp_async<16>(d + f * L::FS + sx, (lin && inx ? a.h[f] : a.old[f]) + (o + gx));
+        }
+    };
+    const double rdx2 = a.rdx * a.rdx, rdy2 = a.rdy * a.rdy, rdz = a.rdz, dt = a.dt;
+    // the pair of field f at a landed level after the horizontal operator
+    auto horizontal = [&](const double* t, double H, double* g) {
+        const double2 c = *reinterpret_cast<const double2*>(t);
+        g[0] = c.x; g[1] = c.y;
+        if (H > 0.) {
+            // rows j-2 .. j+2 of the pair and its neighbours: [2], [3] are the pair
+            double r0[6], rn[4], rs[4];
+            {
+                const double2 w = *reinterpret_cast<const double2*>(t - 2), e = *reinterpret_cast<const double2*>(t + 2);
+                r0[0] = w.x; r0[1] = w.y; r0[2] = c.x; r0[3] = c.y; r0[4] = e.x; r0[5] = e.y;
+                const double2 n = *reinterpret_cast<const double2*>(t + L::FP), q = *reinterpret_cast<const double2*>(t - L::FP);
+                rn[0] = t[L::FP - 1]; rn[1] = n.x; rn[2] = n.y; rn[3] = t[L::FP + 2];
+                rs[0] = t[-L::FP - 1]; rs[1] = q.x; rs[2] = q.y; rs[3] = t[-L::FP + 2];
+            }
+            const double2 nn = *reinterpret_cast<const double2*>(t + 2 * L::FP);
+            const double2 ss = *reinterpret_cast<const double2*>(t - 2 * L::FP);
+            const double cx = -H * rdx2, cy = -H * rdy2;
+            auto lap = [&](double w, double m, double e, double lo, double hi) {
+                return ((e - m) - (m - w)) * cx + ((hi - m) - (m - lo)) * cy;
+            };
+            double d[4];   // first Laplacian at the pair and the points west and east of it
+#pragma unroll
+            for (int q = 0; q < 4; ++q) d[q] = lap(r0[q], r0[q + 1], r0[q + 2], rs[q], rn[q]);
+            const double dn[2] = {lap(rn[0], rn[1], rn[2], c.x, nn.x), lap(rn[1], rn[2], rn[3], c.y, nn.y)};
+            const double ds[2] = {lap(rs[0], rs[1], rs[2], ss.x, c.x), lap(rs[1], rs[2], rs[3], ss.y, c.y)};
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const double m = d[q + 1];
+                g[q] = g[q] + dt * (((d[q + 2] - m) - (m - d[q])) * rdx2 + ((dn[q] - m) - (m - ds[q])) * rdy2);
+            }
+        }
+    };
+    double w[4][5][2];   // levels k-2 .. k+2 of the pair
+    copy_plane(kb - 2);
+    cp_commit();
+    copy_plane(kb - 1);
+    cp_commit();
+    for (int m = kb - 2; m <= ke + 1; ++m) {
+        cp_wait<1>();
+        __syncthreads();   // plane m has landed; plane m-1 is read
+        if (m + 2 <= ke + 1) copy_plane(m + 2);
+        cp_commit();
+        const int k = m - 2;
+        const unsigned g = (unsigned)max(k, 0) * plane + gcol;
+        double2 t0[4], t1[4], t2[4];
+        const bool h1 = a.ab1 != 0.0, h2 = a.ab2 != 0.0;
+        if (k >= kb) {
+#pragma unroll
+            for (int f = 0; f < 4; ++f) {
+                t0[f] = __ldg(reinterpret_cast<const double2*>(a.t0[f] + g));
+                t1[f] = h1 ? __ldg(reinterpret_cast<const double2*>(a.t1[f] + g)) : make_double2(0.0, 0.0);
+                t2[f] = h2 ? __ldg(reinterpret_cast<const double2*>(a.t2[f] + g)) : make_double2(0.0, 0.0);
+            }
+        }
+        const double* pl = ring[(m + 3) % 3][0] + pos;
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) { w[f][q][0] = w[f][q + 1][0]; w[f][q][1] = w[f][q + 1][1]; }
+            // a level outside the interior holds the start-of-step value
+            horizontal(pl + f * L::FS, m >= 0 && m < nz ? a.hmix[f] : 0.0, w[f][4]);
+        }
+        if (k < kb) continue;
+#pragma unroll
+        for (int f = 0; f < 4; ++f) {
+            double o[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                double x = w[f][2][q];
+                const double V = a.vmix[f];
+                if (V > 0.) {
+                    // fluxes between the window's levels; none through a rigid lid or bottom
+                    double f1[4], d2[3];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        f1[j] = a.rigid && (k - 1 + j <= 0 || k - 1 + j >= nz) ? 0.0 : -V * (w[f][j + 1][q] - w[f][j][q]) * rdz;
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) d2[j] = (f1[j + 1] - f1[j]) * rdz;
+                    const double lo = a.rigid && k <= 0 ? 0.0 : (d2[1] - d2[0]) * rdz;
+                    const double hi = a.rigid && k + 1 >= nz ? 0.0 : (d2[2] - d2[1]) * rdz;
+                    x = x + dt * ((hi - lo) * rdz);
+                    if (f == 2 && a.rigid && k == nz - 1) x = 0.0;   // w(:,:,nz:nz+2) = 0 after biharmonic_v(w)
+                }
+                o[q] = x;
+            }
+            if (a.wm_on && (a.wr[f] || a.wi[f])) {
+                const double2 r = a.wr[f] ? __ldg(reinterpret_cast<const double2*>(a.wr[f] + g)) : make_double2(0.0, 0.0);
+                const double2 i = a.wi[f] ? __ldg(reinterpret_cast<const double2*>(a.wi[f] + g)) : make_double2(0.0, 0.0);
+                o[0] = o[0] + dt * (a.wm_c * r.x + a.wm_s * i.x);
+                o[1] = o[1] + dt * (a.wm_c * r.y + a.wm_s * i.y);
+            }
+            const double h = f == 2 ? a.dtw : dt;
+            double tx_ = a.ab0 * t0[f].x, ty_ = a.ab0 * t0[f].y;
+            if (h1) { tx_ = tx_ + a.ab1 * t1[f].x; ty_ = ty_ + a.ab1 * t1[f].y; }
+            if (h2) { tx_ = tx_ + a.ab2 * t2[f].x; ty_ = ty_ + a.ab2 * t2[f].y; }
+            if (active) *reinterpret_cast<double2*>(a.out[f] + g) = make_double2(o[0] + h * tx_, o[1] + h * ty_);
+        }
+    }
+}
+
 // background-flow forcing on the friction-updated state (generic path).
 // set_forcing runs after the in-place friction with no halo exchange, so a
 // neighbour outside the interior still holds its start-of-step value: those
@@ -826,6 +992,28 @@ cudaError_t launch_step(const StepArgs& a, bool fp32_tendencies, cudaStream_t s)
 static inline int grid_for(long n, int threads) {
     long b = (n + threads - 1) / threads;
     return (int)std::min<long>(b, 148L * 16);
+}
+
+// The z chunk minimises waves x (levels + 6): the march loads four planes more
+// than it writes, and starting costs about two.
+cudaError_t launch_friction(const FrictionArgs& a0, cudaStream_t s) {
+    FrictionArgs a = a0;
+    static const int per_sm = [] {
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_friction_ab<8>, kTX / 2 * 8, 0) != cudaSuccess) cudaGetLastError();
+        return n > 0 ? n : 1;
+    }();
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long slots = (long)sms * per_sm, tiles = (long)((a.nx + kTX - 1) / kTX) * ((a.ny + 7) / 8);
+    double best = 1e300;
+    for (int kc = (a.nz + 65534) / 65535; kc <= std::min(a.nz, 64); ++kc) {
+        const double c = (double)((tiles * ((a.nz + kc - 1) / kc) + slots - 1) / slots) * (kc + 6);
+        if (c < best) { best = c; a.kchunk = kc; }
+    }
+    return launch_pdl(k_friction_ab<8>, dim3((a.nx + kTX - 1) / kTX, (a.ny + 7) / 8, (a.nz + a.kchunk - 1) / a.kchunk),
+                      dim3(kTX / 2, 8), 0, s, a);
 }
 
 cudaError_t launch_biharmonic_h(const double* cur, const double* old, double* out, int nx, int ny, int nz,

@@ -115,3 +115,32 @@ def test_periodic_z_solve_in_registers(n, monkeypatch):
         got.append(mm.download(tendencies=False))
     for k in FIELDS + ("p",):
         assert np.array_equal(got[0][k], got[1][k]), k
+
+
+BIHARMONIC = {"all": dict(Ahbi=1e7, Avbi=1e1, Khbi=1e7, Kvbi=1e1), "horizontal": dict(Ahbi=1e7),
+              "vertical": dict(Avbi=1e1, Kvbi=1e1)}
+
+
+@pytest.mark.parametrize("mix", sorted(BIHARMONIC))
+@pytest.mark.parametrize("harmonic", [False, True])
+@pytest.mark.parametrize("n", [(4, 4, 2), (36, 10, 3), (64, 8, 5), (30, 18, 23)])
+@pytest.mark.parametrize("rigid", [True, False])
+def test_biharmonic_in_one_pass(n, harmonic, mix, rigid):
+    """Biharmonic friction, wavemaker and Adams-Bashforth in one kernel: four
+    AB3 steps, the state's correction pending (no harmonic friction) or
+    applied, grids narrower and wider than the tile, odd z chunks."""
+    nz = n[2] if rigid else {2: 2, 3: 4, 5: 6, 23: 24}[n[2]]
+    p = small_params(n[0], n[1], nz, rigid=rigid, **({} if harmonic else FRICTION["none"]), **BIHARMONIC[mix])
+    f = smooth_state(p, seed=37)
+    o, m = _pair(p, f)
+    rng = np.random.default_rng(38)
+    g = {k: cf.halo_fill(a * rng.standard_normal(m.shape)) for k, a in (("u_r", 1e-6), ("u_i", 1e-6), ("b_i", 1e-9))}
+    F = abi.Forcing()
+    F.kind, F.omega = abi.PS3D_FORCE_WAVEMAKER, 5e-4
+    F.u_r, F.u_i, F.b_i = (abi.dptr(g[k]) for k in ("u_r", "u_i", "b_i"))
+    o.set_forcing(F, g)
+    m.set_forcing(abi.PS3D_FORCE_WAVEMAKER, omega=5e-4, **g)
+    o.integrate(4)
+    m.run(4)
+    err = compare_state(m, o)
+    assert max(err.values()) < TOL64, err
