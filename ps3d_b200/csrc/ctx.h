@@ -145,6 +145,7 @@ struct Ctx {
     int win_kbeg = 0, win_kcount = 0, win_kofs = 0, win_nzg = 0;
     bool split_solve = false;
     int kchunk = 8;             // z levels per block of the step kernel
+    int yfused = 0;             // the FP64 pressure solve's y transforms and vertical solve in one kernel (k_ycol)
     bool tune_timing = true;    // false: the autotuner takes cached choices or the defaults, no timing runs
     std::string tuned;          // description of the autotuned choice
     DevBuf twx;
@@ -227,6 +228,7 @@ struct Ctx {
 
     int init(const ps3d_params& prm, int dev, int nbatch = 1, cudaStream_t use_stream = nullptr);
     int autotune();
+    bool ycol_allowed() const, ycol_default() const;
     int model_kchunk() const;   // the step kernel's z chunk by the wave model (engine.cu)
     int advance(int nsteps, bool allow_graph);
     bool graphable() const;

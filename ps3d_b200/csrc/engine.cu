@@ -177,8 +177,10 @@ static std::vector<PlaneArgs> plane_candidates(int nx, int ny, size_t es, const 
     }
     // rows pass + y-lines pass, and its pipelined-rows variant
     for (int im : {1, 2}) {
-        for (int tj : {4, 8, 16, 32}) {
-            if (ny % tj || (im == 1 && tj == 4) || (im == 2 && tj > 16)) continue;
+        for (int tj : {2, 4, 8, 16, 32}) {
+            // rows of fewer than 8 (short runs of the spectra) only where ny
+            // has no larger power of two
+            if (ny % tj || (im == 1 && tj < 8 && ny % (2 * tj) == 0) || (im == 2 && (tj > 16 || tj < 4))) continue;
             // FP32 runs both rows passes in registers (no rows-per-CTA parameter)
             if (im == 1 && es == sizeof(float2) && rows_in_registers(nx, ny) && tj != 16) continue;
             for (int ly : {8, 16, 32}) {
@@ -223,7 +225,8 @@ bool choose_plane_config(int nx, int ny, size_t es, PlaneArgs& a) {
 static bool choose_split_config(int nx, int ny, size_t es, PlaneArgs& a, int impl) {
     for (const PlaneArgs& c : plane_candidates(nx, ny, es, a)) {
         if (c.impl != impl || c.ly != 16) continue;
-        if (c.tj == (impl == 2 ? 8 : 16) || (c.tj == (impl == 2 ? 4 : 8) && ny % (impl == 2 ? 8 : 16))) {
+        const int want = impl == 2 ? 8 : 16;   // the largest power of two up to it that divides ny
+        if (c.tj == want || (c.tj < want && ny % (2 * c.tj))) {
             const FFTPlan px = a.px, py = a.py;
             a = c;
             a.px = px; a.py = py;
@@ -416,6 +419,7 @@ int Ctx::init(const ps3d_params& prm, int dev, int nbatch, cudaStream_t use_stre
     CK(cudaHostGetDevicePointer((void**)&kerr_d, kerr_h, 0));
     pa64.err = kerr_d; pa32.err = kerr_d;
     kchunk = model_kchunk();
+    yfused = ycol_allowed() && pa64.impl >= 1 && ycol_default();
     // reductions
     nred = 148 * 4;
     CK(red_partials.alloc((size_t)nred * 5 * sizeof(double)));
@@ -709,6 +713,19 @@ int Ctx::model_kchunk() const {
     return best;
 }
 
+// the FP64 solve under a rigid lid on the [k][kx][ky] layout, in one grid's
+// whole columns; PS3D_YFUSED=0 keeps the y lines and the vertical solve apart
+bool Ctx::ycol_allowed() const {
+    const char* e = std::getenv("PS3D_YFUSED");
+    return !(e && e[0] == '0') && !mixed && rigid && !split_solve && ycol_fits(nz, ny);
+}
+// Untuned (tiny) grids: fused where every kx has an SM of its own.  Per step,
+// apart and fused: 32x32x16 23.9 and 19.1 us, 48x40x24 28.7 and 21.9 us.
+// Tuned grids take the faster of the two: 96x80x50 51.3 and 43.6 us,
+// 128x128x32 50.9 and 45.7 us, 64x64x32 28.7 and 27.3 us, but 64x128x64 53.4
+// and 54.0 us (a block's 131 KB of spectra leave 33 of 148 SMs at work).
+bool Ctx::ycol_default() const { return (long)nxh * batch <= 148; }
+
 int Ctx::autotune() {
     std::lock_guard<std::mutex> tune_lock(g_tune_mu);
     const char* env = std::getenv("PS3D_AUTOTUNE");
@@ -744,12 +761,14 @@ int Ctx::autotune() {
     // PS3D_TUNE pins a configuration in the cache's format, e.g.
     // "im1,C1,rc8,tj16,ly8,pol2,kc8" (reproducible profiling, no timing runs)
     auto parse = [](const char* str, int* v) {
-        return std::sscanf(str, "im%d,C%d,rc%d,tj%d,ly%d,pol%d,kc%d", &v[0], &v[1], &v[2], &v[3], &v[4], &v[5],
-                           &v[6]) == 7;
+        v[7] = 0;   // optional: the fused y transforms and vertical solve
+        return std::sscanf(str, "im%d,C%d,rc%d,tj%d,ly%d,pol%d,kc%d,yf%d", &v[0], &v[1], &v[2], &v[3], &v[4], &v[5],
+                           &v[6], &v[7]) >= 7;
     };
     if (const char* pin = std::getenv("PS3D_TUNE")) {
         int v[8];
         if (parse(pin, v) && apply(v[0], v[1], v[2], v[3], v[4], v[5], v[6])) {
+            yfused = v[7] && ycol_allowed();
             tuned = std::string("pinned:") + pin;
             return PS3D_OK;
         }
@@ -759,6 +778,7 @@ int Ctx::autotune() {
     if (it != tune_cache().end()) {
         int v[8];
         if (parse(it->second.c_str(), v) && apply(v[0], v[1], v[2], v[3], v[4], v[5], v[6])) {
+            yfused = v[7] && ycol_allowed();
             tuned = std::string("cached:") + it->second;
             return PS3D_OK;
         }
@@ -767,18 +787,23 @@ int Ctx::autotune() {
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
+    // the best of five runs, or of three times three short ones (launches start
+    // on a grid of about 2 us, coarser than the differences between small kernels)
     auto timeit = [&](auto&& fn) -> float {
         float best = 1e30f;
         if (fn() != PS3D_OK) return best;
         if (cudaStreamSynchronize(stream) != cudaSuccess) { cudaGetLastError(); return best; }
-        for (int r = 0; r < 5; ++r) {
+        int reps = 1;
+        for (int r = 0; r < (reps > 1 ? 4 : 6); ++r) {
             cudaEventRecord(e0, stream);
-            if (fn() != PS3D_OK) return 1e30f;
+            for (int q = 0; q < reps; ++q)
+                if (fn() != PS3D_OK) return 1e30f;
             cudaEventRecord(e1, stream);
             if (cudaEventSynchronize(e1) != cudaSuccess) { cudaGetLastError(); return 1e30f; }
             float ms = 0.f;
             cudaEventElapsedTime(&ms, e0, e1);
-            best = std::min(best, ms);
+            if (r == 0) reps = ms < 0.1f ? 3 : 1;
+            else best = std::min(best, ms / reps);
         }
         return best;
     };
@@ -808,6 +833,31 @@ int Ctx::autotune() {
     }
     bestpa.batch = 1;
     pa = bestpa;
+    // the whole solve of a field of zeros: with the winner as it is, and with
+    // the y transforms and the vertical solve in one kernel between the rows
+    // passes of every rows shape
+    yfused = 0;
+    if (ycol_allowed() && plane_force != 0) {
+        const long long l0 = launches;
+        auto solve = [&]() -> int { return poisson_once((double*)p.p, 0.0, true); };
+        float tb = timeit(solve);
+        yfused = 1;
+        int bestyf = 0;
+        for (const PlaneArgs& cand : plane_candidates(nx, ny, sizeof(double2), pa)) {
+            if (cand.impl != 1 || (plane_force > 1) || cand.ly != 16) continue;   // no y-lines pass: ly does not matter
+            for (int pol = 0; pol < 3; ++pol) {
+                pa = cand;
+                plans_of(pol, pa);
+                pa.batch = 1;
+                const float t = timeit(solve);
+                if (t < tb) { tb = t; bestpa = pa; bestpol = pol; bestyf = 1; }
+            }
+        }
+        pa = bestpa;
+        yfused = bestyf;
+        pending = false;
+        launches = l0;
+    }
     // step kernel z chunk: powers of two and the chunk of the wave model
     std::vector<int> kcs = {1, 2, 4, 8, 16, 32};
     {
@@ -848,8 +898,8 @@ int Ctx::autotune() {
     cudaEventDestroy(e1);
     CK(cudaStreamSynchronize(stream));
     char val[128];
-    std::snprintf(val, sizeof val, "im%d,C%d,rc%d,tj%d,ly%d,pol%d,kc%d", pa.impl, pa.C, pa.row_chunk, pa.tj, pa.ly,
-                  bestpol, kchunk);
+    std::snprintf(val, sizeof val, "im%d,C%d,rc%d,tj%d,ly%d,pol%d,kc%d,yf%d", pa.impl, pa.C, pa.row_chunk, pa.tj, pa.ly,
+                  bestpol, kchunk, yfused);
     tuned = val;
     tune_cache_store(key, val);
     return PS3D_OK;
@@ -945,6 +995,7 @@ int Ctx::poisson_once(double* out, double beta, bool lazy, const double* pc) {
     const bool f32 = mixed;
     PlaneArgs a = f32 ? pa32 : pa64;
     a.batch = batch;
+    a.yfused = yfused;
     a.mode = pc ? 2 : 0;
     a.u = field(0); a.v = field(1); a.w = field(2);
     a.pc = pc; a.dtp = P.dt; a.dtwp = P.dt / P.dsqr; a.rigid = rigid;
@@ -961,6 +1012,10 @@ int Ctx::poisson_once(double* out, double beta, bool lazy, const double* pc) {
         c.fxa = 1.0 / (P.dz * P.dz) / P.dsqr;
         c.dz2dsqr = P.dz * P.dz * P.dsqr;
         LAUNCH(PS3D_K_VSOLVE, launch_colsolve(a, c, stream));
+    } else if (rigid && a.yfused) {
+        c.fxa = 1.0 / (P.dz * P.dz) / P.dsqr;
+        c.dz2dsqr = P.dz * P.dz * P.dsqr;
+        LAUNCH(PS3D_K_VSOLVE, launch_ycol(a, c, stream));
     } else if (rigid) {
         c.fxa = 1.0 / (P.dz * P.dz) / P.dsqr;
         c.dz2dsqr = P.dz * P.dz * P.dsqr;
@@ -971,6 +1026,7 @@ int Ctx::poisson_once(double* out, double beta, bool lazy, const double* pc) {
     }
     PlaneArgs b = f32 ? pa32 : pa64;
     b.batch = batch;
+    b.yfused = yfused;
     b.spec = FS.p;
     b.out = out;
     b.beta = beta;
@@ -1803,9 +1859,9 @@ int ps3d_describe(ps3d_ctx* ctx, char* buf, int len) {
     const Ctx& C = ctx->impl;
     const ps3d::PlaneArgs& pa = C.mixed ? C.pa32 : C.pa64;
     std::snprintf(buf, len, "grid=%dx%dx%d precision=%s batch=%d plane_impl=%s plane_cluster=%d row_chunk=%d tj=%d ly=%d "
-                  "fft_x=%d stages fft_y=%d stages kchunk=%d vmode=%s tuned=%s", C.nx, C.ny, C.nz, C.refine_full ? "mixed_refined" : C.mixed ? "mixed" : "fp64",
+                  "fft_x=%d stages fft_y=%d stages kchunk=%d yfused=%d vmode=%s tuned=%s", C.nx, C.ny, C.nz, C.refine_full ? "mixed_refined" : C.mixed ? "mixed" : "fp64",
                   C.batch, pa.impl == 2 ? "pipe+lines" : pa.ysplit ? "rows+colsolve" : pa.impl ? "rows+lines" : "cluster", pa.C, pa.row_chunk, pa.tj, pa.ly, pa.px.nst, pa.py.nst,
-                  C.kchunk, !C.rigid ? "z-fft" : C.vmode_fft ? "fft" : "dense", C.tuned.empty() ? "default" : C.tuned.c_str());
+                  C.kchunk, C.yfused, !C.rigid ? "z-fft" : C.vmode_fft ? "fft" : "dense", C.tuned.empty() ? "default" : C.tuned.c_str());
     return PS3D_OK;
 }
 

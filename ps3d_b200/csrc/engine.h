@@ -135,6 +135,9 @@ struct PlaneArgs {
     // vertical solve are then one kernel, k_colsolve (launch_colsolve)
     int ysplit;
     FFTPlan pyh;                   // ysplit: the half-length y plan (length ny/2)
+    // implementation 1 or 2, FP64: the y transforms and the rigid-lid vertical
+    // solve are one kernel, k_ycol (launch_ycol)
+    int yfused;
     int zrev;                      // the rows passes walk the planes top down (set by the launchers)
 };
 // spectral layout of a plane configuration: 0 [k][ky][kx], 1 [k][kx][ky]
@@ -212,6 +215,9 @@ int thomas_threads(int nz);
 // (FP32 spectra); p: the forward plane arguments (scale, half-length plan)
 cudaError_t launch_colsolve(const PlaneArgs& p, const ColumnArgs& c, cudaStream_t s);
 bool colsolve_fits(int nz, int ny);
+// the same on the natural layout, FP64 spectra, one block per kx (PlaneArgs::yfused)
+cudaError_t launch_ycol(const PlaneArgs& p, const ColumnArgs& c, cudaStream_t s);
+bool ycol_fits(int nz, int ny);
 bool colsolve2_fits(int nz, int ny);   // the two-CTA cluster form (half the levels per CTA)
 // periodic z solve; zsolve_fits(nz, fp32) false: too tall for a block's shared memory
 cudaError_t launch_zsolve(const ColumnArgs& a, bool fp32, cudaStream_t s);

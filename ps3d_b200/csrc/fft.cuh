@@ -126,12 +126,19 @@ PS3D_HD void small_dft(T* v, int sign) {
 struct StageSplit {
     int line0, bfly0, bstep;
 };
-__device__ __forceinline__ StageSplit stage_split(int nslots) {
+__device__ __forceinline__ StageSplit stage_split(int nslots, int nthreads) {
     StageSplit s;
     s.line0 = threadIdx.x % nslots;
     s.bfly0 = threadIdx.x / nslots;
-    s.bstep = blockDim.x / nslots;
+    s.bstep = nthreads / nslots;
     return s;
+}
+
+// barrier of the block, or (NTHR > 0) of its first NTHR threads alone
+template <int NTHR>
+__device__ __forceinline__ void fft_sync() {
+    if constexpr (NTHR > 0) asm volatile("bar.sync 1, %0;\n" ::"n"(NTHR) : "memory");
+    else __syncthreads();
 }
 
 template <int RAD, bool DIT, typename R>
@@ -196,12 +203,14 @@ __device__ __forceinline__ void fft_stage(cpx<R>* buf, int ld, int nlines, const
 // kernels built with MAXR = 8 hold fewer registers and run more blocks per
 // SM, and only take plans without radix-16 stages.  NSLOTS > 0 selects the
 // fixed-line split (NSLOTS must divide the block size, nlines <= NSLOTS is
-// passed at run time); 0 splits (butterfly, line) items.
-template <bool DIT, typename R, int MAXR = 16, bool FIXED = false>
+// passed at run time); 0 splits (butterfly, line) items.  NTHR > 0: only the
+// block's first NTHR threads call it (fixed-line split only).
+template <bool DIT, typename R, int MAXR = 16, bool FIXED = false, int NTHR = 0>
 __device__ void fft_batch(cpx<R>* buf, int ld, int nlines, const FFTPlan& P, int sign, const cpx<R>* tw,
                           int nslots = 0) {
-    __syncthreads();
-    const StageSplit sp = stage_split(FIXED ? nslots : 1);
+    static_assert(NTHR == 0 || FIXED, "a part of the block: fixed-line split");
+    fft_sync<NTHR>();
+    const StageSplit sp = stage_split(FIXED ? nslots : 1, NTHR > 0 ? NTHR : blockDim.x);
     for (int s0 = 0; s0 < P.nst; ++s0) {
         const int st = DIT ? s0 : P.nst - 1 - s0;
         const int Lp = P.lp[st];
@@ -216,7 +225,7 @@ __device__ void fft_batch(cpx<R>* buf, int ld, int nlines, const FFTPlan& P, int
                 break;
             default: break;
         }
-        __syncthreads();
+        fft_sync<NTHR>();
     }
 }
 

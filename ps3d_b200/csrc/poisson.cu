@@ -999,6 +999,212 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kCsThreads, 2) k_col
     }
 }
 
+// The y transforms and the rigid-lid vertical solve of one kx in one block, in
+// FP64 on the natural layout [k][kx][ky], for grids whose launches are shorter
+// than the gaps between them: three kernels and four trips of the spectra
+// become one and two.  The block holds its nz x ny spectra as [j][k] with an
+// odd pitch (the FFT's lines are the levels, the solve's columns the j, which
+// stay digit-reversed between the two transforms).  The elimination is
+// k_thomas2's, two-ended; the right-hand side is overwritten by d' and d'' in
+// FP64, so the way back forms nothing again.
+// Bound by latency: a load, two FFTs of two or three stages, the elimination
+// and a store follow one another in the block.  The serial chain of reciprocal
+// pivots does not depend on the data: ny extra threads form it while the
+// others load and transform, which leaves one multiply-add a level.
+// Measured times and the sizes it is taken for: Ctx::ycol_default.
+constexpr int kYcThreads = 256, kYcKC = 8;
+
+PS3D_HD size_t ycol_smem(int nz, int ny) {
+    return align16((size_t)ny * (nz | 1) * sizeof(double2)) + align16((size_t)((nz + 1) / 2 + 1) * ny * sizeof(double)) +
+           plan_tables_bytes(ny, sizeof(double2));
+}
+bool ycol_fits(int nz, int ny) {
+    return nz <= kYcThreads && ny <= 256 && ycol_smem(nz, ny) <= 227 * 1024 - 64;
+}
+
+struct YColArgs {
+    int nz, ny, nxh;
+    double2* spec;
+    long sM;
+    FFTPlan py;
+    double scale;
+    const double *hkx, *hky;
+    double fxa, dz2dsqr;
+    int nslots;                    // lines the FFTs' threads are dealt to: nz rounded up to a power of two
+    FastDiv fd_ny;
+    int l2hint;
+};
+
+template <int MAXR>
+__global__ void __launch_bounds__(kYcThreads + 256, 1) k_ycol(const YColArgs a) {
+    using T = double2;
+    constexpr int NT = kYcThreads, KC = kYcKC;
+    pdl_trigger();
+    extern __shared__ __align__(16) unsigned char yc_raw[];
+    const int nz = a.nz, ny = a.ny, nxh = a.nxh, ld = nz | 1;
+    const int H = (nz + 1) / 2, Bc = nz - H, m = H - 1, jb = Bc - 1;
+    T* buf = reinterpret_cast<T*>(yc_raw);                                                         // [j][k]
+    // [jj][j]: reciprocal pivots of levels 0 .. H-1, then that of the 2x2 solve in the middle
+    double* piv = reinterpret_cast<double*>(yc_raw + align16((size_t)ny * ld * sizeof(T)));
+    unsigned char* tail = yc_raw + align16((size_t)ny * ld * sizeof(T)) + align16((size_t)(H + 1) * ny * sizeof(double));
+    const int inst = blockIdx.x / nxh, kx = blockIdx.x - inst * nxh;
+    const int tid = threadIdx.x;
+    const double fxa = a.fxa;
+    if (tid >= NT) {
+        // the pivots: r(0) = 1/b(1), r(jj) = 1/(b - cp(jj-1) a), cp = c r
+        const int p = tid - NT;
+        if (p < ny) {
+            const double ks = a.hkx[kx] + a.hky[__ldg(a.py.ipos + p)];
+            const double bmid = -ks - 2 * fxa;
+            double r = ks > 0 ? 1.0 / (-ks - fxa) : 0.0, cp = fxa * r, cp_jb = cp;
+            piv[p] = r;
+            if (ks > 0) {
+                for (int jj = 1; jj < H; ++jj) {
+                    r = rcp_newton(bmid - cp * fxa);
+                    cp = fxa * r;
+                    piv[jj * ny + p] = r;
+                    if (jj == jb) cp_jb = cp;
+                }
+                piv[H * ny + p] = 1.0 / (1.0 - cp * cp_jb);
+            }
+        }
+        __syncthreads();
+        return;
+    }
+    const PlanTables<double> ty = [&] {   // stage_plan by the first NT threads
+        T* t = reinterpret_cast<T*>(tail);
+        int* q0 = reinterpret_cast<int*>(tail + align16((size_t)ny * sizeof(T)));
+        int* q1 = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(q0) + align16((size_t)ny * sizeof(int)));
+        for (int e = tid; e < ny; e += NT) {
+            t[e] = __ldg(a.py.tw + e);
+            q0[e] = __ldg(a.py.pos + e);
+            q1[e] = __ldg(a.py.ipos + e);
+        }
+        return PlanTables<double>{t, q0, q1};
+    }();
+    pdl_wait();   // inputs written by the preceding kernels
+    T* g = a.spec + (long)inst * a.sM + (long)kx * ny;
+    const long ls = (long)nxh * ny;   // level stride
+    const unsigned long long pk = pol_keep(a.l2hint);
+    const int total = nz * ny;
+    constexpr int LB = 8;
+    for (int t0 = tid; t0 < total; t0 += LB * NT) {
+        T v[LB];
+#pragma unroll
+        for (int q = 0; q < LB; ++q) {
+            const int t = t0 + q * NT;
+            if (t < total) {
+                const int k = (int)fdiv(t, a.fd_ny), j = t - k * ny;
+                v[q] = ld_l2(&g[(long)k * ls + j], pk);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < LB; ++q) {
+            const int t = t0 + q * NT;
+            if (t < total) {
+                const int k = (int)fdiv(t, a.fd_ny), j = t - k * ny;
+                buf[j * ld + k] = cscale(v[q], a.scale);
+            }
+        }
+    }
+    fft_batch<false, double, MAXR, true, NT>(buf, ld, nz, a.py, -1, ty.tw, a.nslots);   // synchronises before and after
+    __syncthreads();   // the pivots are formed
+    for (int c = tid; c < 2 * ny; c += NT) {
+        const int p = c >> 1;
+        double* col = reinterpret_cast<double*>(buf + (size_t)p * ld) + (c & 1);   // level k at col[2 k]
+        const double* pv = piv + p;                                              // pivot level jj at pv[jj ny]
+        if (!(pv[0] != 0.0)) {
+            // (0,0): p(1) = 0, p(2) = f(1) dz^2 dsqr, p(k+1) = 2p(k) - p(k-1) + f(k) dz^2 dsqr
+            double x0 = 0.0, x1 = 0.0, fprev = 0.0;
+            for (int k0 = 0; k0 < nz; k0 += KC) {
+                double d[KC];
+#pragma unroll
+                for (int q = 0; q < KC; ++q) d[q] = k0 + q < nz ? col[2 * (k0 + q)] : 0.0;
+#pragma unroll
+                for (int q = 0; q < KC; ++q)
+                    if (k0 + q < nz) {
+                        const double xk = k0 + q == 0 ? 0.0 : 2 * x1 - x0 + fprev * a.dz2dsqr;
+                        fprev = d[q];
+                        x0 = x1; x1 = xk;
+                        col[2 * (k0 + q)] = xk;
+                    }
+            }
+            continue;
+        }
+        double* bot = col + 2 * (nz - 1);   // bottom chain: level nz-1-jj at bot[-2 jj]
+        double dp = 0.0, dq = 0.0, r = 0.0, r_jb = 0.0;
+        for (int jc = 0; jc < H; jc += KC) {
+            double dt[KC], db[KC], rr[KC];
+#pragma unroll
+            for (int q = 0; q < KC; ++q) {
+                const int jj = jc + q;
+                dt[q] = jj < H ? col[2 * jj] : 0.0;
+                db[q] = jj < Bc ? bot[-2 * jj] : 0.0;
+                rr[q] = jj < H ? pv[jj * ny] : 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < KC; ++q) {
+                const int jj = jc + q;
+                if (jj < H) {   // d' = (d - d' a) r, d' = 0 before the first level
+                    r = rr[q];
+                    const double cp = fxa * r;
+                    dp = fma(-cp, dp, dt[q] * r);
+                    col[2 * jj] = dp;
+                    if (jj < Bc) {
+                        dq = fma(-cp, dq, db[q] * r);
+                        bot[-2 * jj] = dq;
+                        r_jb = r;
+                    }
+                }
+            }
+        }
+        // the two halves meet, then back substitution outward
+        double xt = (dp - fxa * r * dq) * pv[H * ny];
+        double xb = dq - fxa * r_jb * xt;
+        col[2 * m] = xt;
+        bot[-2 * jb] = xb;
+        for (int jc = (m - 1) / KC * KC; jc >= 0 && m > 0; jc -= KC) {
+            double dt[KC], db[KC], cc[KC];
+#pragma unroll
+            for (int q = 0; q < KC; ++q) {
+                const int jj = jc + q;
+                dt[q] = jj < m ? col[2 * jj] : 0.0;
+                db[q] = jj < jb ? bot[-2 * jj] : 0.0;
+                cc[q] = jj < m ? fxa * pv[jj * ny] : 0.0;
+            }
+#pragma unroll
+            for (int q = KC - 1; q >= 0; --q) {
+                const int jj = jc + q;
+                if (jj < m) { xt = fma(-cc[q], xt, dt[q]); col[2 * jj] = xt; }
+                if (jj < jb) { xb = fma(-cc[q], xb, db[q]); bot[-2 * jj] = xb; }
+            }
+        }
+    }
+    fft_batch<true, double, MAXR, true, NT>(buf, ld, nz, a.py, +1, ty.tw, a.nslots);
+    for (int t = tid; t < total; t += NT) {
+        const int k = (int)fdiv(t, a.fd_ny), j = t - k * ny;
+        st_l2(&g[(long)k * ls + j], buf[j * ld + k], pk);
+    }
+}
+
+cudaError_t launch_ycol(const PlaneArgs& p, const ColumnArgs& c, cudaStream_t s) {
+    if (!ycol_fits(c.nz, c.ny)) return cudaErrorInvalidValue;
+    YColArgs a{};
+    a.nz = c.nz; a.ny = c.ny; a.nxh = c.nxh;
+    a.spec = reinterpret_cast<double2*>(c.spec); a.sM = c.sM;
+    a.py = p.py;
+    a.scale = p.scale;
+    a.hkx = c.hkx; a.hky = c.hky;
+    a.fxa = c.fxa; a.dz2dsqr = c.dz2dsqr;
+    a.nslots = 1;
+    while (a.nslots < c.nz) a.nslots *= 2;
+    a.fd_ny = make_fastdiv(c.ny);
+    a.l2hint = l2hint_mode();
+    const dim3 g((unsigned)(c.nxh * std::max(1, c.batch))), b(kYcThreads + (c.ny + 31) / 32 * 32);
+    const size_t sm = ycol_smem(c.nz, c.ny);
+    return plan_max_radix(p.py) >= 16 ? launch_pdl(k_ycol<16>, g, b, sm, s, a) : launch_pdl(k_ycol<8>, g, b, sm, s, a);
+}
+
 bool colsolve_fits(int nz, int ny) {
     return ny % 16 == 0 && colsolve_smem(nz, ny) <= 227 * 1024 - 64;
 }
@@ -1962,9 +2168,13 @@ static cudaError_t launch_split_m(const PlaneArgs& a, bool fwd, cudaStream_t s) 
     cudaError_t e = cudaSuccess;
     if (fwd && a.impl == 2 && a.mode != 2) {
         e = launch_pipe<R, MX>(a, s);
-        if (e != cudaSuccess) return e;
+        if (e != cudaSuccess || a.yfused) return e;
         if (!ylines_reg<R>(ay, -1, a.scale, s, &e))
             e = launch_pdl(k_ylines<R, MY>, glines, dim3(kPlaneThreads), sml, s, ay, -1, a.scale);
+    } else if (fwd && a.yfused) {   // the y transforms run inside k_ycol
+        if (!rows_reg<R>(a, true, s, &e)) e = launch_pdl(k_rows_fwd<R, MX>, grows, dim3(kPlaneThreads), smr, s, a);
+    } else if (a.yfused) {
+        if (!rows_reg<R>(a, false, s, &e)) e = launch_pdl(k_rows_inv<R, MX>, grows, dim3(kPlaneThreads), smr, s, a);
     } else if (fwd && a.ysplit) {   // the y transforms run inside k_colsolve
         if (!rows_reg<R>(a, true, s, &e)) return cudaErrorInvalidValue;
     } else if (a.ysplit) {
@@ -2061,6 +2271,8 @@ static cudaError_t setup_t() {
     if ((e = max_dynamic_smem(k_thomas2<R, false, true>))) return e;
     if ((e = max_dynamic_smem(k_thomas2<R, true, true>))) return e;
     if ((e = max_dynamic_smem(k_colsolve))) return e;
+    if ((e = max_dynamic_smem(k_ycol<16>))) return e;
+    if ((e = max_dynamic_smem(k_ycol<8>))) return e;
     if ((e = max_dynamic_smem(k_colsolve2))) return e;
     if ((e = max_dynamic_smem(k_thomas<R, true>))) return e;
     if ((e = max_dynamic_smem(k_thomas<R, false>))) return e;

@@ -144,3 +144,24 @@ def test_biharmonic_in_one_pass(n, harmonic, mix, rigid):
     m.run(4)
     err = compare_state(m, o)
     assert max(err.values()) < TOL64, err
+
+
+@pytest.mark.parametrize("n", [(16, 4, 2), (16, 10, 3), (36, 20, 17), (32, 64, 32), (24, 80, 50), (16, 150, 65)])
+def test_fused_y_transforms_and_vertical_solve(n, monkeypatch):
+    """The FP64 y transforms and rigid-lid vertical solve in one block per kx
+    (odd and even nz, more columns than threads) against the oracle, and
+    against the separate kernels."""
+    p = small_params(*n, rigid=True)
+    f = random_state(p, seed=39)
+    o = Oracle(p)
+    load_oracle(o, f)
+    o.pressure_solver()
+    monkeypatch.setenv("PS3D_AUTOTUNE", "0")
+    for form in ("1", "0"):
+        monkeypatch.setenv("PS3D_YFUSED", form)
+        m = Model(p)
+        m.upload(**{k: f[k] for k in FIELDS})
+        m.pressure_solver()
+        assert f"yfused={form}" in m.describe()
+        err = compare_state(m, o)
+        assert max(err.values()) < TOL_KERNEL, (form, err)
