@@ -101,6 +101,106 @@ __device__ __forceinline__ double2 plane_source_pair(const PlaneArgs& a, const d
     return d;
 }
 
+// The same for a run of rows j0 .. j0+n-1 at one pair m, walking along y: the
+// corrected v and the pressure of a row are the next row's southern ones, every
+// offset is 32-bit within the instance, and the periodic neighbours along x
+// are found once.  LB rows' loads go out together; store(r, d) takes row j0+r.
+// Formed point by point, 157 of a pair's 272 instructions in the rows pass were
+// index arithmetic; forward transforms, before and after: 256x256x128 FP64 99.4
+// and 92.5 us, 512x256x64 94.4 and 86.6 us mixed, 128x128x64 25.5 and 20.0 us
+// mixed.  LB is chosen against registers: two rows in flight in FP64 (four
+// spill the 80 registers of three blocks, 117 us), one with the pressure's
+// seven further loads (two cost the FP32 register pass blocks: 108.9 against
+// 86.6 us at 512x256x64), two where a thread walks only 8 rows (nx = 128).
+template <int MODE, int LB, class Store>
+__device__ __forceinline__ void rows_source(const PlaneArgs& a, const double* au, const double* av, const double* aw,
+                                              const double* src, int k, int j0, int n, int m,
+                                              unsigned long long pol, const Store& store) {
+    const int nx = a.nx, ny = a.ny, nz = a.nz;
+    const unsigned plane = (unsigned)nx * ny;
+    auto ld2 = [&](const double* f, unsigned o) { return ldg_l2(reinterpret_cast<const double2*>(f + o), pol); };
+    const unsigned col = (unsigned)k * plane + 2 * m;
+    if constexpr (MODE == 1) {
+        for (int r0 = 0; r0 < n; r0 += 4) {
+            double2 d[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (r0 + q < n) d[q] = ld2(src, col + (unsigned)(j0 + r0 + q) * nx);
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (r0 + q < n) store(r0 + q, d[q]);
+        }
+        return;
+    }
+    const double* pc = MODE == 2 ? a.pc + (au - a.u) : nullptr;   // same instance offset as the fields
+    const int west = 2 * m - 1 < 0 ? nx - 1 : -1, east = 2 * m + 2 >= nx ? 2 - nx : 2;
+    const unsigned low = (unsigned)wrap(k - 1, nz) * plane + 2 * m, up = (unsigned)wrap(k + 1, nz) * plane + 2 * m;
+    const int kg = k + a.kofs, nzg = a.nzg ? a.nzg : nz;   // global level (z-slabs)
+    const bool lid = a.rigid && kg == nzg - 1, floor_ = a.rigid && kg == 0;   // the level below the floor is the lid
+    const double dt = a.dtp, dtw = a.dtwp;
+    double2 vm = ld2(av, col + (unsigned)wrap(j0 - 1, ny) * nx), p0 = make_double2(0.0, 0.0);
+    if constexpr (MODE == 2) {
+        const double2 ps = ld2(pc, col + (unsigned)wrap(j0 - 1, ny) * nx);
+        p0 = ld2(pc, col + (unsigned)j0 * nx);
+        vm.x = vm.x - dt * (p0.x - ps.x) * a.rdy;
+        vm.y = vm.y - dt * (p0.y - ps.y) * a.rdy;
+    }
+#pragma unroll 1
+    for (int r0 = 0; r0 < n; r0 += LB) {
+        double2 uu[LB], vv[LB], ww[LB], wm[LB], pn[LB], pd[LB], pu[LB];
+        double um[LB], pw[LB], pe[LB];
+#pragma unroll
+        for (int q = 0; q < LB; ++q) {
+            if (r0 + q < n) {
+                const int j = j0 + r0 + q;
+                const unsigned row = (unsigned)j * nx, g = col + row;
+                uu[q] = ld2(au, g);
+                um[q] = ldg_l2(au + (g + west), pol);
+                vv[q] = ld2(av, g);
+                ww[q] = ld2(aw, g);
+                wm[q] = ld2(aw, low + row);
+                if constexpr (MODE == 2) {
+                    pn[q] = ld2(pc, col + (unsigned)(j + 1 == ny ? 0 : j + 1) * nx);
+                    pw[q] = ldg_l2(pc + (g + west), pol);
+                    pe[q] = ldg_l2(pc + (g + east), pol);
+                    pd[q] = ld2(pc, low + row);
+                    pu[q] = ld2(pc, up + row);
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < LB; ++q) {
+            if (r0 + q < n) {
+                if constexpr (MODE == 2) {
+                    // u - dt grad p at the points the divergence reads (pressure_solver.f90:98-110)
+                    um[q] = um[q] - dt * (p0.x - pw[q]) * a.rdx;
+                    uu[q].x = uu[q].x - dt * (p0.y - p0.x) * a.rdx;
+                    uu[q].y = uu[q].y - dt * (pe[q] - p0.y) * a.rdx;
+                    vv[q].x = vv[q].x - dt * (pn[q].x - p0.x) * a.rdy;
+                    vv[q].y = vv[q].y - dt * (pn[q].y - p0.y) * a.rdy;
+                    if (lid) {
+                        ww[q].x = 0.0; ww[q].y = 0.0;
+                    } else {
+                        ww[q].x = ww[q].x - dtw * (pu[q].x - p0.x) * a.rdz;
+                        ww[q].y = ww[q].y - dtw * (pu[q].y - p0.y) * a.rdz;
+                    }
+                    if (floor_) {
+                        wm[q].x = 0.0; wm[q].y = 0.0;
+                    } else {
+                        wm[q].x = wm[q].x - dtw * (p0.x - pd[q].x) * a.rdz;
+                        wm[q].y = wm[q].y - dtw * (p0.y - pd[q].y) * a.rdz;
+                    }
+                    p0 = pn[q];
+                }
+                double2 d;
+                d.x = ((uu[q].x - um[q]) * a.rdx + (vv[q].x - vm.x) * a.rdy + (ww[q].x - wm[q].x) * a.rdz) * a.rdt;
+                d.y = ((uu[q].y - uu[q].x) * a.rdx + (vv[q].y - vm.y) * a.rdy + (ww[q].y - wm[q].y) * a.rdz) * a.rdt;
+                vm = vv[q];
+                store(r0 + q, d);
+            }
+        }
+    }
+}
 // exp(-2 pi i t / nx), t = 0..nx/2, staged in the working precision
 template <typename R>
 __device__ cpx<R>* stage_twx(const PlaneArgs& a, unsigned char* dst) {
@@ -1419,7 +1519,7 @@ __global__ void __launch_bounds__(kZRegThreads, 4) k_zsolve_reg(const ColumnArgs
 // before their shared-memory stores, so each thread keeps several loads in
 // flight.
 // ---------------------------------------------------------------------------
-template <typename R, int MAXR>
+template <typename R, int MAXR, int MODE>
 __global__ void __launch_bounds__(kPlaneThreads, plane_min_blocks<MAXR>()) k_rows_fwd(const PlaneArgs a) {
     pdl_trigger();
     pdl_wait();   // inputs written by the preceding kernels
@@ -1444,35 +1544,26 @@ __global__ void __launch_bounds__(kPlaneThreads, plane_min_blocks<MAXR>()) k_row
     const double* av = a.v + ioff;
     const double* aw = a.w + ioff;
     const double* asrc = a.src ? a.src + ioff : nullptr;
-    constexpr int LB = 2;
-    const int total = tj * n2;
-    for (int t0 = threadIdx.x; t0 < total; t0 += LB * blockDim.x) {
-        double2 d[LB];
-#pragma unroll
-        for (int q = 0; q < LB; ++q) {
-            const int t = t0 + q * blockDim.x;
-            if (t < total) {
-                const int rr = (int)fdiv(t, a.fd_n2), m = t - rr * n2;
-                d[q] = plane_source_pair(a, au, av, aw, asrc, k, jb + rr, m, pfield);
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < LB; ++q) {
-            const int t = t0 + q * blockDim.x;
-            if (t < total) {
-                const int rr = (int)fdiv(t, a.fd_n2), m = t - rr * n2;
-                buf[m * ld + rr] = mk<R>((R)d[q].x, (R)d[q].y);
-            }
-        }
+    // a thread keeps one pair m and walks a run of the block's rows
+    {
+        const int groups = max(1, min(tj, kPlaneThreads / n2)), per = (tj + groups - 1) / groups;
+        const int gr = n2 <= kPlaneThreads ? (int)fdiv(threadIdx.x, a.fd_n2) : 0;
+        const int r0 = gr * per, nr = min(per, tj - r0);
+        if (gr < groups && nr > 0)
+            for (int m = threadIdx.x - gr * n2; m < n2; m += kPlaneThreads)
+                rows_source<MODE, MODE == 2 ? 1 : 2>(a, au, av, aw, asrc, k, jb + r0, nr, m, pfield, [&](int r, double2 d) {
+                    buf[m * ld + r0 + r] = mk<R>((R)d.x, (R)d.y);
+                });
     }
     fft_batch<false, R, MAXR, true>(buf, ld, tj, a.px, -1, tx.tw, tj);   // its first barrier also orders the tables
-    T* spec = reinterpret_cast<T*>(a.spec) + (long)inst * a.sM + (long)kl * nxh * ny;
-    for (int t = threadIdx.x; t < tj * (n2 + 1); t += blockDim.x) {
-        const int kx = (int)fdiv(t, a.fd_tj), rr = t - kx * tj;
+    // tj divides the block: a thread keeps one row and steps through kx
+    T* spec = reinterpret_cast<T*>(a.spec) + (long)inst * a.sM + (long)kl * nxh * ny + jb;
+    const int kx0 = (int)fdiv(threadIdx.x, a.fd_tj), rr = threadIdx.x - kx0 * tj, kstep = kPlaneThreads / tj;
+    for (int kx = kx0; kx <= n2; kx += kstep) {
         const int k1 = (kx == n2) ? 0 : kx;
         const int k2 = (kx == 0) ? 0 : n2 - kx;
-        st_l2(&spec[(long)kx * ny + jb + rr], r2c_unpack<R>(buf[tx.pos[k1] * ld + rr], buf[tx.pos[k2] * ld + rr], twx[kx]),
-              pkeep);
+        st_l2(&spec[(unsigned)kx * (unsigned)ny + rr],
+              r2c_unpack<R>(buf[tx.pos[k1] * ld + rr], buf[tx.pos[k2] * ld + rr], twx[kx]), pkeep);
     }
 }
 
@@ -1771,7 +1862,7 @@ __device__ __forceinline__ int rowreg_row(int jb_block, int r, int ny) {
     return jb_block * (TJ / 2) + (r < TJ / 2 ? r : ny / 2 + r - TJ / 2);
 }
 
-template <typename R, int N1, int N2, bool YS>
+template <typename R, int N1, int N2, bool YS, int MODE>
 __global__ void __launch_bounds__(RowReg<N1, N2, R>::NT) k_rows_fwd_reg(const PlaneArgs a) {
     pdl_trigger();
     pdl_wait();   // inputs written by the preceding kernels
@@ -1794,23 +1885,17 @@ __global__ void __launch_bounds__(RowReg<N1, N2, R>::NT) k_rows_fwd_reg(const Pl
     const long ioff = (long)inst * a.sN;
     const double* asrc = a.src ? a.src + ioff : nullptr;
     const T* tw = reinterpret_cast<const T*>(sizeof(R) == 8 ? (const void*)a.px.tw : (const void*)a.px.twf);
-    // z = s(2m) + i s(2m+1) of the block's rows, formed by all lanes with m
-    // fastest (coalesced, LB points in flight per lane) into each row's tile
-    constexpr int LB = 4;
-    static_assert((N * TJ) % (LB * G::NT) == 0, "source batches");
-    for (int t0 = threadIdx.x; t0 < N * TJ; t0 += LB * G::NT) {
-        double2 d[LB];
-#pragma unroll
-        for (int q = 0; q < LB; ++q) {
-            const int t = t0 + q * G::NT;
-            d[q] = plane_source_pair(a, a.u + ioff, a.v + ioff, a.w + ioff, asrc, k,
-                                     rowreg_row<TJ, YS>(blockIdx.x, t / N, ny), t % N, pfield);
-        }
-#pragma unroll
-        for (int q = 0; q < LB; ++q) {
-            const int t = t0 + q * G::NT;
-            tb[(t / N) * G::LS + t % N] = mk<R>((R)d[q].x, (R)d[q].y);
-        }
+    // z = s(2m) + i s(2m+1) of the block's rows into each row's tile: a thread
+    // keeps one m (consecutive threads, consecutive m) and walks a run of rows
+    {
+        constexpr int GR = G::NT / N, per = TJ / GR;   // groups of threads, rows of each
+        static_assert(G::NT % N == 0 && TJ % GR == 0 && (!YS || per <= TJ / 2 || GR == 1), "rows of a group");
+        const int m = threadIdx.x % N, r0 = threadIdx.x / N * per;
+        constexpr int run = YS && per > TJ / 2 ? TJ / 2 : per;   // rows that are neighbours in y
+#pragma unroll 1
+        for (int rb = r0; rb < r0 + per; rb += run)
+            rows_source<MODE, MODE == 2 ? (N <= 64 ? 2 : 1) : 4>(a, a.u + ioff, a.v + ioff, a.w + ioff, asrc, k, rowreg_row<TJ, YS>(blockIdx.x, rb, ny), run, m,
+                              pfield, [&](int r, double2 d) { tb[(rb + r) * G::LS + m] = mk<R>((R)d.x, (R)d.y); });
     }
     __syncthreads();
     T* t1 = tb + row * G::LS;   // this row's tile: the source, then the transpose
@@ -2132,18 +2217,20 @@ static cudaError_t launch_rows_reg_t(const PlaneArgs& a, bool fwd, cudaStream_t 
     const dim3 g(a.ny / G::TJ, (a.kcount ? a.kcount : a.nz) * std::max(1, a.batch));
     const size_t sm = G::elems * sizeof(cpx<R>);
     if (a.ysplit) {
-        if (fwd) return launch_pdl(k_rows_fwd_reg<R, N1, N2, true>, g, dim3(G::NT), sm, s, a);
+        if (fwd && a.mode == 0) return launch_pdl(k_rows_fwd_reg<R, N1, N2, true, 0>, g, dim3(G::NT), sm, s, a);
+        if (fwd && a.mode == 1) return launch_pdl(k_rows_fwd_reg<R, N1, N2, true, 1>, g, dim3(G::NT), sm, s, a);
+        if (fwd) return launch_pdl(k_rows_fwd_reg<R, N1, N2, true, 2>, g, dim3(G::NT), sm, s, a);
         return launch_pdl(k_rows_inv_reg<R, N1, N2, true>, g, dim3(G::NT), sm, s, a);
     }
-    if (fwd) return launch_pdl(k_rows_fwd_reg<R, N1, N2, false>, g, dim3(G::NT), sm, s, a);
+    if (fwd && a.mode == 0) return launch_pdl(k_rows_fwd_reg<R, N1, N2, false, 0>, g, dim3(G::NT), sm, s, a);
+    if (fwd && a.mode == 1) return launch_pdl(k_rows_fwd_reg<R, N1, N2, false, 1>, g, dim3(G::NT), sm, s, a);
+    if (fwd) return launch_pdl(k_rows_fwd_reg<R, N1, N2, false, 2>, g, dim3(G::NT), sm, s, a);
     return launch_pdl(k_rows_inv_reg<R, N1, N2, false>, g, dim3(G::NT), sm, s, a);
-    return cudaGetLastError();
 }
 // The register rows pass when nx/2 has a two-factor split, else false.  The
-// FP64 forward pass keeps the staged kernel: its register form needs ~92
-// registers for the 16 source points of a lane and runs 5 blocks per SM,
-// too few to cover the six loads per point (112.8 vs 105.4 us for the
-// forward transform at 256x256x128); in FP32 it runs 7 (87 vs 100 us).
+// FP64 forward pass keeps the staged kernel (92.8 us for the forward transform
+// at 256x256x128, 99.0 us with the register form's 94 registers and five
+// blocks an SM).
 template <typename R>
 static bool rows_reg(const PlaneArgs& a, bool fwd, cudaStream_t s, cudaError_t* e) {
     if (fwd && sizeof(R) == 8) return false;
@@ -2154,6 +2241,13 @@ static bool rows_reg(const PlaneArgs& a, bool fwd, cudaStream_t s, cudaError_t* 
         case 512: *e = launch_rows_reg_t<R, 16, 16>(a, fwd, s); return true;
         default: return false;
     }
+}
+
+template <typename R, int MX>
+static cudaError_t launch_rows_fwd(const PlaneArgs& a, dim3 g, size_t sm, cudaStream_t s) {
+    if (a.mode == 0) return launch_pdl(k_rows_fwd<R, MX, 0>, g, dim3(kPlaneThreads), sm, s, a);
+    if (a.mode == 1) return launch_pdl(k_rows_fwd<R, MX, 1>, g, dim3(kPlaneThreads), sm, s, a);
+    return launch_pdl(k_rows_fwd<R, MX, 2>, g, dim3(kPlaneThreads), sm, s, a);
 }
 
 template <typename R, int MX, int MY>
@@ -2172,7 +2266,7 @@ static cudaError_t launch_split_m(const PlaneArgs& a, bool fwd, cudaStream_t s) 
         if (!ylines_reg<R>(ay, -1, a.scale, s, &e))
             e = launch_pdl(k_ylines<R, MY>, glines, dim3(kPlaneThreads), sml, s, ay, -1, a.scale);
     } else if (fwd && a.yfused) {   // the y transforms run inside k_ycol
-        if (!rows_reg<R>(a, true, s, &e)) e = launch_pdl(k_rows_fwd<R, MX>, grows, dim3(kPlaneThreads), smr, s, a);
+        if (!rows_reg<R>(a, true, s, &e)) e = launch_rows_fwd<R, MX>(a, grows, smr, s);
     } else if (a.yfused) {
         if (!rows_reg<R>(a, false, s, &e)) e = launch_pdl(k_rows_inv<R, MX>, grows, dim3(kPlaneThreads), smr, s, a);
     } else if (fwd && a.ysplit) {   // the y transforms run inside k_colsolve
@@ -2180,7 +2274,7 @@ static cudaError_t launch_split_m(const PlaneArgs& a, bool fwd, cudaStream_t s) 
     } else if (a.ysplit) {
         if (!rows_reg<R>(a, false, s, &e)) return cudaErrorInvalidValue;
     } else if (fwd) {
-        if (!rows_reg<R>(a, true, s, &e)) e = launch_pdl(k_rows_fwd<R, MX>, grows, dim3(kPlaneThreads), smr, s, a);
+        if (!rows_reg<R>(a, true, s, &e)) e = launch_rows_fwd<R, MX>(a, grows, smr, s);
         if (e != cudaSuccess) return e;
         if (!ylines_reg<R>(ay, -1, a.scale, s, &e))
             e = launch_pdl(k_ylines<R, MY>, glines, dim3(kPlaneThreads), sml, s, ay, -1, a.scale);
@@ -2243,7 +2337,9 @@ static cudaError_t setup_m() {
     if ((e = cudaFuncSetAttribute(k_plane_inv<R, MAXR>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm))) return e;
     if ((e = cudaFuncSetAttribute(k_plane_fwd<R, MAXR>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))) return e;
     if ((e = cudaFuncSetAttribute(k_plane_inv<R, MAXR>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))) return e;
-    if ((e = cudaFuncSetAttribute(k_rows_fwd<R, MAXR>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm))) return e;
+    if ((e = cudaFuncSetAttribute(k_rows_fwd<R, MAXR, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm))) return e;
+    if ((e = cudaFuncSetAttribute(k_rows_fwd<R, MAXR, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm))) return e;
+    if ((e = cudaFuncSetAttribute(k_rows_fwd<R, MAXR, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm))) return e;
     if ((e = cudaFuncSetAttribute(k_rows_inv<R, MAXR>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm))) return e;
     if ((e = cudaFuncSetAttribute(k_ylines<R, MAXR>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm))) return e;
     if ((e = max_dynamic_smem(k_rows_fwd_pipe<R, MAXR>))) return e;
@@ -2256,9 +2352,15 @@ static cudaError_t setup_t() {
     if ((e = max_dynamic_smem(k_ylines_reg<R, 16, 8>))) return e;
     if ((e = max_dynamic_smem(k_ylines_reg<R, 16, 16>))) return e;
 #define PS3D_ROWS_SETUP(YS)                                                   \
-    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 8, 8, YS>))) return e;       \
-    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 16, 8, YS>))) return e;      \
-    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 16, 16, YS>))) return e;     \
+    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 8, 8, YS, 0>))) return e;     \
+    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 8, 8, YS, 1>))) return e;     \
+    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 8, 8, YS, 2>))) return e;     \
+    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 16, 8, YS, 0>))) return e;    \
+    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 16, 8, YS, 1>))) return e;    \
+    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 16, 8, YS, 2>))) return e;    \
+    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 16, 16, YS, 0>))) return e;   \
+    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 16, 16, YS, 1>))) return e;   \
+    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 16, 16, YS, 2>))) return e;   \
     if ((e = max_dynamic_smem(k_rows_inv_reg<R, 8, 8, YS>))) return e;       \
     if ((e = max_dynamic_smem(k_rows_inv_reg<R, 16, 8, YS>))) return e;      \
     if ((e = max_dynamic_smem(k_rows_inv_reg<R, 16, 16, YS>))) return e;
