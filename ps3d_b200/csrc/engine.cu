@@ -1902,12 +1902,16 @@ const char* ps3d_strerror(int status) {
 }  // extern "C"
 
 namespace ps3d {
-bool pdl_enabled() {
-    static const bool on = [] {
+bool pdl_launch(dim3 grid, cudaStream_t s) {
+    static const int mode = [] {
         const char* e = std::getenv("PS3D_PDL");
-        return e && e[0] == '1';
+        return e ? (e[0] == '1' ? 1 : 0) : -1;
     }();
-    return on;
+    if (mode >= 0) return mode == 1;
+    if ((long)grid.x * grid.y * grid.z > 148) return false;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) { cudaGetLastError(); return false; }
+    return st == cudaStreamCaptureStatusNone;
 }
 
 // Records the last failing CUDA call; printed to stderr when PS3D_VERBOSE is set.

@@ -8,12 +8,15 @@
 namespace ps3d {
 
 // Launch with programmatic stream serialization (see pdl_trigger/pdl_wait):
-// only for kernels that call pdl_wait before reading their inputs.  Off by
-// default (ordinary full dependencies; griddepcontrol.wait then returns at
-// once): measured on a B200 at 256x256x128, the programmatic overlap made
-// the step 95 us slower in both precisions, eager or in CUDA graphs.
-// PS3D_PDL=1 turns it on.
-bool pdl_enabled();
+// only for kernels that call pdl_wait before reading their inputs (a launch
+// without it has ordinary full dependencies; griddepcontrol.wait then returns
+// at once).  Taken for eager launches of at most a block per SM, whose start
+// is then hidden behind the kernel before: a host stepping a 32x32x16 grid
+// call by call takes 1.01 ms per 24 steps without and 0.86 ms with it.  Not
+// taken inside CUDA graphs (64x64x32: 31.3 us a step without, 33.0 with it) nor
+// for grids that fill the GPU (256x256x128: 95 us a step slower).  PS3D_PDL=0
+// never, =1 always.
+bool pdl_launch(dim3 grid, cudaStream_t s);
 template <typename... P, typename... A>
 inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                               A&&... args) {
@@ -26,7 +29,7 @@ inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = pdl_launch(grid, s) ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<A&&>(args)...);
 }
 
