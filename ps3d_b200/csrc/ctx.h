@@ -229,7 +229,8 @@ struct Ctx {
     int init(const ps3d_params& prm, int dev, int nbatch = 1, cudaStream_t use_stream = nullptr);
     int autotune();
     bool ycol_allowed() const, ycol_default() const;
-    int model_kchunk() const;   // the step kernel's z chunk by the wave model (engine.cu)
+    // the step kernel's z chunk by the wave model (engine.cu); adds its next best ones to *more
+    int model_kchunk(std::vector<int>* more = nullptr) const;
     int advance(int nsteps, bool allow_graph);
     bool graphable() const;
     int capture_graph(GraphSlot& slot);

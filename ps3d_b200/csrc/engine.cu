@@ -196,8 +196,7 @@ static std::vector<PlaneArgs> plane_candidates(int nx, int ny, size_t es, const 
     return out;
 }
 
-// Default cluster shape of the plane kernels for one element size (also the
-// shape of ps3d_pressure_solve_noalloc's plane kernels).
+// Default cluster shape of the plane kernels for one element size.
 bool choose_plane_config(int nx, int ny, size_t es, PlaneArgs& a) {
     const int nxh = nx / 2 + 1;
     for (int pass = 0; pass < 2; ++pass) {
@@ -221,8 +220,8 @@ bool choose_plane_config(int nx, int ny, size_t es, PlaneArgs& a) {
 }
 
 // Default shape of the rows + y-lines plane kernels (implementation 1 or 2)
-// for one element size.
-static bool choose_split_config(int nx, int ny, size_t es, PlaneArgs& a, int impl) {
+// for one element size (also of ps3d_pressure_solve_noalloc).
+bool choose_split_config(int nx, int ny, size_t es, PlaneArgs& a, int impl) {
     for (const PlaneArgs& c : plane_candidates(nx, ny, es, a)) {
         if (c.impl != impl || c.ly != 16) continue;
         const int want = impl == 2 ? 8 : 16;   // the largest power of two up to it that divides ny
@@ -693,8 +692,8 @@ static void tune_cache_store(const std::string& k, const std::string& v) {
 // about three levels of its march (measured 6.5 us + 1.25 us a level at
 // 32x32x16), and a last wave that is nearly empty costs a whole one.  At
 // 32x32x16 it gives 1 (64 blocks, 7.5 us; 34 us as one chunk of 16), at
-// 64x64x32 2, at 256x256x128 12 (6.3 waves of 444 blocks).
-int Ctx::model_kchunk() const {
+// 64x64x32 2, at 256x256x128 26 (2.9 waves of 444 blocks).
+int Ctx::model_kchunk(std::vector<int>* more) const {
     StepArgs q{};
     q.harm_uvw = (P.Ah > 0. || P.Av > 0.); q.harm_b = (P.Kh > 0. || P.Kv > 0.);
     q.wm_on = (fkind & PS3D_FORCE_WAVEMAKER) ? 1 : 0;
@@ -737,7 +736,7 @@ int Ctx::autotune() {
     cudaDeviceProp prop;
     CK(cudaGetDeviceProperties(&prop, dev));
     char key[384];
-    std::snprintf(key, sizeof key, "%s|%dx%dx%d|p%d|r%d|b%d|i%d|s2", prop.name, nx, ny, nz, (int)mixed, (int)rigid, batch,
+    std::snprintf(key, sizeof key, "%s|%dx%dx%d|p%d|r%d|b%d|i%d|s3", prop.name, nx, ny, nz, (int)mixed, (int)rigid, batch,
                   plane_force);
     for (char* c = key; *c; ++c) if (*c == ' ') *c = '_';
     const bool f32 = mixed;
@@ -802,7 +801,7 @@ int Ctx::autotune() {
             if (cudaEventSynchronize(e1) != cudaSuccess) { cudaGetLastError(); return 1e30f; }
             float ms = 0.f;
             cudaEventElapsedTime(&ms, e0, e1);
-            if (r == 0) reps = ms < 0.1f ? 3 : 1;
+            if (r == 0) reps = ms < 0.5f ? 3 : 1;
             else best = std::min(best, ms / reps);
         }
         return best;
@@ -858,12 +857,11 @@ int Ctx::autotune() {
         pending = false;
         launches = l0;
     }
-    // step kernel z chunk: powers of two and the chunk of the wave model
+    // step kernel z chunk: powers of two and the best chunks of the wave model
+    // (at 256x256x128 the mixed kernel takes 214 us with 24 levels, 216 with
+    // the model's first, 26, and 221 with 32; FP64 234 with 13, 236 with 26)
     std::vector<int> kcs = {1, 2, 4, 8, 16, 32};
-    {
-        const int mkc = model_kchunk();
-        if (std::find(kcs.begin(), kcs.end(), mkc) == kcs.end()) kcs.push_back(mkc);
-    }
+    model_kchunk(&kcs);
     float bestk = 1e30f;
     int bestkc = kchunk;
     for (int kc : kcs) {

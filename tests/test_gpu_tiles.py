@@ -165,3 +165,25 @@ def test_fused_y_transforms_and_vertical_solve(n, monkeypatch):
         assert f"yfused={form}" in m.describe()
         err = compare_state(m, o)
         assert max(err.values()) < TOL_KERNEL, (form, err)
+
+
+@pytest.mark.parametrize("rigid", [True, False])
+def test_noalloc_projection_shapes(rigid):
+    """ps3d_pressure_solve_noalloc on grids of each route (y transforms with
+    the vertical solve; y lines of their own where there are more kx than SMs;
+    rows passes of 2 to 16 rows), one after the other and back again, so that
+    each call finds another grid's tables."""
+    grids = [(48, 40, 24), (6, 10, 4), (300, 16, 8), (32, 54, 20), (48, 40, 24), (8, 250, 16), (200, 2, 30)]
+    for seed, n in enumerate(grids):
+        p = small_params(*n, rigid=rigid)
+        f = random_state(p, seed=40 + seed)
+        o = Oracle(p)
+        load_oracle(o, f)
+        o.pressure_solver()
+        got = _noalloc(p, f)
+        pn = np.linalg.norm(cf.interior(o.field("p")))
+        for k, d in (("p", None), ("u", p.dx), ("v", p.dy), ("w", p.dz)):
+            want = cf.interior(o.field(k))
+            # a velocity carries p's rounding times dt over its grid distance
+            tol = TOL_KERNEL + (8 * np.finfo(float).eps * p.dt / d * pn / np.linalg.norm(want) if d else 0.0)
+            assert np.linalg.norm(got[k] - want) <= tol * np.linalg.norm(want), (n, k)
