@@ -702,22 +702,26 @@ int Ctx::model_kchunk(std::vector<int>* more) const {
     const long slots = (long)sms * step_resident(q, hist32);
     const long tiles = (long)((nx + 31) / 32) * ((ny + 7) / 8) * std::max(1, batch);
     const int levels = win_kcount ? win_kcount : nz;
-    double bestc = 1e300;
-    int best = 1;
+    std::vector<std::pair<double, int>> cost;   // of the smallest chunk for each number of chunks
     for (int kc = 1; kc <= std::min(levels, 48); ++kc) {
-        const long blocks = tiles * ((levels + kc - 1) / kc);
-        const double c = (double)((blocks + slots - 1) / slots) * (kc + 3);
-        if (c < bestc * (1 - 1e-9)) { bestc = c; best = kc; }
+        const long n = (levels + kc - 1) / kc, blocks = tiles * n;
+        if (kc > 1 && (levels + kc - 2) / (kc - 1) == n) continue;
+        cost.push_back({(double)((blocks + slots - 1) / slots) * (kc + 3), kc});
     }
-    return best;
+    std::stable_sort(cost.begin(), cost.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
+    if (more)
+        for (size_t q = 0; q < cost.size() && q < 6; ++q)
+            if (std::find(more->begin(), more->end(), cost[q].second) == more->end()) more->push_back(cost[q].second);
+    return cost[0].second;
 }
 
 // the FP64 solve under a rigid lid on the [k][kx][ky] layout, in one grid's
 // whole columns; PS3D_YFUSED=0 keeps the y lines and the vertical solve apart
-bool Ctx::ycol_allowed() const {
+bool ycol_enabled(int nz, int ny) {
     const char* e = std::getenv("PS3D_YFUSED");
-    return !(e && e[0] == '0') && !mixed && rigid && !split_solve && ycol_fits(nz, ny);
+    return !(e && e[0] == '0') && ycol_fits(nz, ny);
 }
+bool Ctx::ycol_allowed() const { return !mixed && rigid && !split_solve && ycol_enabled(nz, ny); }
 // Untuned (tiny) grids: fused where every kx has an SM of its own.  Per step,
 // apart and fused: 32x32x16 23.9 and 19.1 us, 48x40x24 28.7 and 21.9 us.
 // Tuned grids take the faster of the two: 96x80x50 51.3 and 43.6 us,

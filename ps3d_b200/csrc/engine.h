@@ -207,6 +207,8 @@ cudaError_t plane_setup(bool fp32);
 // default one-cluster-per-plane shape for element size es (false: no shape
 // fits the shared memory of a block)
 bool choose_plane_config(int nx, int ny, size_t es, PlaneArgs& a);
+// default rows + y-lines shape (implementation 1 or 2; false: none fits the grid)
+bool choose_split_config(int nx, int ny, size_t es, PlaneArgs& a, int impl);
 cudaError_t launch_plane_fwd(const PlaneArgs& a, bool fp32, cudaStream_t s);
 cudaError_t launch_plane_inv(const PlaneArgs& a, bool fp32, cudaStream_t s);
 int plane_max_clusters(const PlaneArgs& a, bool fp32, bool fwd);
@@ -221,6 +223,7 @@ bool colsolve_fits(int nz, int ny);
 // the same on the natural layout, FP64 spectra, one block per kx (PlaneArgs::yfused)
 cudaError_t launch_ycol(const PlaneArgs& p, const ColumnArgs& c, cudaStream_t s);
 bool ycol_fits(int nz, int ny);
+bool ycol_enabled(int nz, int ny);   // ycol_fits, unless PS3D_YFUSED=0
 bool colsolve2_fits(int nz, int ny);   // the two-CTA cluster form (half the levels per CTA)
 // periodic z solve; zsolve_fits(nz, fp32) false: too tall for a block's shared memory
 cudaError_t launch_zsolve(const ColumnArgs& a, bool fp32, cudaStream_t s);

@@ -32,26 +32,50 @@ namespace ps3d {
 constexpr long kMaxSpectral = 1L << 20;     // complex doubles in the spectral scratch
 constexpr int kMaxLen = 1024;               // longest FFT / axis the tables cover
 
-// table layout inside g_tables (in doubles)
-constexpr long kTwX = 0;                          // tw (length nx/2), double2
-constexpr long kTwY = kTwX + 2L * kMaxLen;        // tw (length ny), double2
-constexpr long kTwZ = kTwY + 2L * kMaxLen;        // tw (length nz), double2
-constexpr long kTwR = kTwZ + 2L * kMaxLen;        // exp(-2 pi i t/nx), t = 0..nx/2, double2
-constexpr long kHkx = kTwR + 2L * (kMaxLen + 1);  // hat_ksqr(kx)
-constexpr long kHky = kHkx + kMaxLen + 1;         // hat_ksqr(ky)
-constexpr long kHkz = kHky + kMaxLen;             // hat_ksqr(kz)/dsqr
-constexpr long kPos = kHkz + kMaxLen;             // int tables start here (6 x kMaxLen ints)
-constexpr long kTableDoubles = kPos + 3L * kMaxLen;
+// table layout inside g_tables (offsets in doubles), packed for the grid of
+// the call: a call copies what its grid uses (4 KB at 48x40x24, of 90 KB)
+struct TableLayout {
+    long twx, twy, twz, twr, hkx, hky, hkz, pos, total;
+    TableLayout(int nx, int ny, int nz, bool rigid) {
+        const long nxh = nx / 2 + 1, zz = rigid ? 0 : nz;
+        twx = 0;                                       // tw (length nx/2), double2
+        twy = twx + 2 * (nx / 2);                      // tw (length ny), double2
+        twz = twy + 2L * ny;                           // tw (length nz), double2
+        twr = twz + 2 * zz;                            // exp(-2 pi i t/nx), t = 0..nx/2, double2
+        hkx = twr + 2 * nxh;                           // hat_ksqr(kx)
+        hky = hkx + nxh;                               // hat_ksqr(ky)
+        hkz = hky + ny;                                // hat_ksqr(kz)/dsqr
+        pos = hkz + zz;                                // int tables: pos and ipos of each plan
+        total = pos + (nx / 2) + ny + zz;
+    }
+};
+constexpr long kTableDoubles = 14L * kMaxLen + 16;    // total at nx/2 = ny = nz = kMaxLen: 14 x 1024 + 3
 
 static __device__ __align__(256) double2 g_spectral[kMaxSpectral];
 static __device__ __align__(256) double g_tables[kTableDoubles];
 
+// what the tables depend on
+struct TableKey {
+    int nx, ny, nz, rigid;
+    double Lx, Ly, Lz, dx, dy, dz, dsqr;
+    bool operator==(const TableKey& o) const {
+        return nx == o.nx && ny == o.ny && nz == o.nz && rigid == o.rigid && Lx == o.Lx && Ly == o.Ly && Lz == o.Lz &&
+               dx == o.dx && dy == o.dy && dz == o.dz && dsqr == o.dsqr;
+    }
+};
+
 // device addresses of the static arrays, looked up once per device, and the
-// host image of the tables (static, so a call allocates no host memory either)
+// host image of the tables (static, so a call allocates no host memory either).
+// The image and its plans stay for the next call of the same grid: a host
+// program projects one grid again and again, and their sines cost more than
+// the copy does.
 struct StaticArrays {
     double2* spectral = nullptr;
     double* tables = nullptr;
     bool ready = false;
+    bool built = false;
+    TableKey key{};
+    FFTPlan px{}, py{}, pz{};
     double img[kTableDoubles];
 };
 static std::mutex g_mu;   // held for a whole call
@@ -76,8 +100,7 @@ static int static_arrays(int dev, StaticArrays*& out) {
 }
 
 // host construction of one FFT plan's tables into the staging image
-static bool plan_into(int n, double* img, long tw_off, long pos_off, long ipos_off, FFTPlan& P,
-                      const double* dev_tables) {
+static bool plan_into(int n, double* img, long tw_off, long int_off, FFTPlan& P, const double* dev_tables) {
     int r[64];
     int nr = 0;
     int m = n;
@@ -88,7 +111,8 @@ static bool plan_into(int n, double* img, long tw_off, long pos_off, long ipos_o
     while (m % 3 == 0) { r[nr++] = 3; m /= 3; }
     while (m % 5 == 0) { r[nr++] = 5; m /= 5; }
     if (m != 1 || n > kMaxLen || nr > kMaxStages) return false;
-    int* ip = reinterpret_cast<int*>(img + kPos);
+    int* pos = reinterpret_cast<int*>(img + int_off);
+    int* ipos = pos + n;
     for (int t = 0; t < n; ++t) {
         long tt = t;
         double c, s;
@@ -104,8 +128,6 @@ static bool plan_into(int n, double* img, long tw_off, long pos_off, long ipos_o
         img[tw_off + 2 * t] = c;
         img[tw_off + 2 * t + 1] = -s;
     }
-    int* pos = ip + ipos_off;   // scratch: overwritten by the inverse table below
-    int* ipos = ip + ipos_off;
     for (int t = 0; t < n; ++t) {
         int v = t, len = n, p = 0;
         for (int st = nr - 1; st >= 0; --st) {
@@ -116,8 +138,7 @@ static bool plan_into(int n, double* img, long tw_off, long pos_off, long ipos_o
         }
         pos[t] = p;
     }
-    for (int t = 0; t < n; ++t) ip[pos_off + t] = pos[t];
-    for (int t = 0; t < n; ++t) ipos[ip[pos_off + t]] = t;
+    for (int t = 0; t < n; ++t) ipos[pos[t]] = t;
     P.n = n;
     P.nst = nr;
     int acc = 1;
@@ -128,9 +149,8 @@ static bool plan_into(int n, double* img, long tw_off, long pos_off, long ipos_o
     }
     P.tw = reinterpret_cast<const double2*>(dev_tables + tw_off);
     P.twf = nullptr;
-    const int* dev_int = reinterpret_cast<const int*>(dev_tables + kPos);
-    P.pos = dev_int + pos_off;
-    P.ipos = dev_int + ipos_off;
+    P.pos = reinterpret_cast<const int*>(dev_tables + int_off);
+    P.ipos = P.pos + n;
     return true;
 }
 
@@ -176,48 +196,59 @@ PS3D_API int ps3d_pressure_solve_noalloc(const ps3d_params* prm, double* u, doub
     cudaStream_t s = (cudaStream_t)stream;
     // tables: built on the host into the static image, copied into g_tables
     double* img = sa->img;
-    std::memset(img, 0, sizeof(sa->img));
-    FFTPlan px{}, py{}, pz{};
-    if (!plan_into(nx / 2, img, kTwX, 0, kMaxLen, px, sa->tables)) return PS3D_ERR_BADPARAM;
-    if (!plan_into(ny, img, kTwY, 2 * kMaxLen, 3 * kMaxLen, py, sa->tables)) return PS3D_ERR_BADPARAM;
-    if (!rigid && !plan_into(nz, img, kTwZ, 4 * kMaxLen, 5 * kMaxLen, pz, sa->tables)) return PS3D_ERR_BADPARAM;
-    const double pi = std::acos(0.0) * 2.0;
-    for (int t = 0; t < nxh; ++t) {
-        long tt = t;
-        double c, sn;
-        if ((8 * tt) % nx == 0) {
-            static const double r2 = 0.70710678118654752440084436210484904;
-            const double cc[8] = {1, r2, 0, -r2, -1, -r2, 0, r2};
-            const double ss[8] = {0, r2, 1, r2, 0, -r2, -1, -r2};
-            c = cc[(8 * tt) / nx]; sn = ss[(8 * tt) / nx];
-        } else {
-            const long double a = 2.0L * 3.14159265358979323846264338327950288L * (long double)tt / (long double)nx;
-            c = (double)cosl(a); sn = (double)sinl(a);
+    const TableLayout T(nx, ny, nz, rigid);
+    const TableKey key{nx, ny, nz, rigid, P.Lx, P.Ly, P.Lz, P.dx, P.dy, P.dz, P.dsqr};
+    FFTPlan &px = sa->px, &py = sa->py, &pz = sa->pz;
+    if (!sa->built || !(sa->key == key)) {
+        sa->built = false;
+        px = FFTPlan{}; py = FFTPlan{}; pz = FFTPlan{};
+        if (!plan_into(nx / 2, img, T.twx, T.pos, px, sa->tables)) return PS3D_ERR_BADPARAM;
+        if (!plan_into(ny, img, T.twy, T.pos + nx / 2, py, sa->tables)) return PS3D_ERR_BADPARAM;
+        if (!rigid && !plan_into(nz, img, T.twz, T.pos + nx / 2 + ny, pz, sa->tables)) return PS3D_ERR_BADPARAM;
+        const double pi = std::acos(0.0) * 2.0;
+        for (int t = 0; t < nxh; ++t) {
+            long tt = t;
+            double c, sn;
+            if ((8 * tt) % nx == 0) {
+                static const double r2 = 0.70710678118654752440084436210484904;
+                const double cc[8] = {1, r2, 0, -r2, -1, -r2, 0, r2};
+                const double ss[8] = {0, r2, 1, r2, 0, -r2, -1, -r2};
+                c = cc[(8 * tt) / nx]; sn = ss[(8 * tt) / nx];
+            } else {
+                const long double a = 2.0L * 3.14159265358979323846264338327950288L * (long double)tt / (long double)nx;
+                c = (double)cosl(a); sn = (double)sinl(a);
+            }
+            img[T.twr + 2 * t] = c;
+            img[T.twr + 2 * t + 1] = -sn;
         }
-        img[kTwR + 2 * t] = c;
-        img[kTwR + 2 * t + 1] = -sn;
-    }
-    auto hat = [](double k, double d) { return 2.0 * (1.0 - std::cos(k * d)) / (d * d); };
-    for (int i = 1; i <= nxh; ++i) img[kHkx + i - 1] = hat(2 * (i - 1) * pi / P.Lx, P.dx);
-    for (int j = 1; j <= ny; ++j) {
-        const double ky = j <= (ny + 1) / 2 ? 2 * (j - 1) * pi / P.Ly : -(2 * (ny - j + 1) * pi / P.Ly);
-        img[kHky + j - 1] = hat(ky, P.dy);
-    }
-    if (!rigid)
-        for (int k = 1; k <= nz; ++k) {
-            const double kz = k <= (nz + 1) / 2 ? 2 * (k - 1) * pi / P.Lz : -(2 * (nz - k + 1) * pi / P.Lz);
-            img[kHkz + k - 1] = hat(kz, P.dz) / P.dsqr;
+        auto hat = [](double k, double d) { return 2.0 * (1.0 - std::cos(k * d)) / (d * d); };
+        for (int i = 1; i <= nxh; ++i) img[T.hkx + i - 1] = hat(2 * (i - 1) * pi / P.Lx, P.dx);
+        for (int j = 1; j <= ny; ++j) {
+            const double ky = j <= (ny + 1) / 2 ? 2 * (j - 1) * pi / P.Ly : -(2 * (ny - j + 1) * pi / P.Ly);
+            img[T.hky + j - 1] = hat(ky, P.dy);
         }
-    // plane-kernel shape: the engine's default one-cluster-per-plane shape
+        if (!rigid)
+            for (int k = 1; k <= nz; ++k) {
+                const double kz = k <= (nz + 1) / 2 ? 2 * (k - 1) * pi / P.Lz : -(2 * (nz - k + 1) * pi / P.Lz);
+                img[T.hkz + k - 1] = hat(kz, P.dz) / P.dsqr;
+            }
+        sa->key = key;
+        sa->built = true;
+    }
+    // plane-kernel shape: the engine's defaults (rows passes with the y lines
+    // or, where every kx gets an SM, with the y transforms and the vertical
+    // solve in one kernel; one cluster per plane where no rows shape fits)
     PlaneArgs a{};
     a.nx = nx; a.ny = ny; a.nz = nz; a.nxh = nxh;
     a.px = px; a.py = py;
-    a.twx = reinterpret_cast<const double2*>(sa->tables + kTwR);
+    a.twx = reinterpret_cast<const double2*>(sa->tables + T.twr);
     a.rdx = 1.0 / P.dx; a.rdy = 1.0 / P.dy; a.rdz = 1.0 / P.dz;
     a.batch = 1; a.sN = (long)nx * ny * nz; a.sM = (long)nxh * ny * nz;
     if (!choose_plane_config(nx, ny, sizeof(double2), a)) return PS3D_ERR_TOOLARGE;
     a.impl = 0;
-    if ((e = cudaMemcpyAsync(sa->tables, img, sizeof(sa->img), cudaMemcpyHostToDevice, s)) != cudaSuccess) return fail(e);
+    if (choose_split_config(nx, ny, sizeof(double2), a, 1)) a.yfused = rigid && nxh <= 148 && ycol_enabled(nz, ny);
+    if ((e = cudaMemcpyAsync(sa->tables, img, T.total * sizeof(double), cudaMemcpyHostToDevice, s)) != cudaSuccess)
+        return fail(e);
     PlaneArgs f = a;
     f.mode = 0; f.u = u; f.v = v; f.w = w;
     f.rdt = 1.0 / P.dt;
@@ -227,12 +258,12 @@ PS3D_API int ps3d_pressure_solve_noalloc(const ps3d_params* prm, double* u, doub
     ColumnArgs c{};
     c.nx = nx; c.ny = ny; c.nz = nz; c.nxh = nxh; c.spec = sa->spectral;
     c.batch = 1; c.sM = a.sM;
-    c.hkx = sa->tables + kHkx; c.hky = sa->tables + kHky; c.hkz = sa->tables + kHkz;
+    c.hkx = sa->tables + T.hkx; c.hky = sa->tables + T.hky; c.hkz = sa->tables + T.hkz;
     c.layout = spectral_layout(a);
     if (rigid) {
         c.fxa = 1.0 / (P.dz * P.dz) / P.dsqr;
         c.dz2dsqr = P.dz * P.dz * P.dsqr;
-        if ((e = launch_thomas(c, false, s)) != cudaSuccess) return fail(e);
+        if ((e = a.yfused ? launch_ycol(f, c, s) : launch_thomas(c, false, s)) != cudaSuccess) return fail(e);
     } else {
         c.pz = pz; c.scale = P.dz; c.op = 0;
         if ((e = launch_zsolve(c, false, s)) != cudaSuccess) return fail(e);

@@ -8,6 +8,7 @@ from ps3d_b200 import abi
 from ps3d_b200 import configs as cf
 from ps3d_b200.model import Model
 from oracle.binding import Oracle
+from tests.test_zz_no_alloc import _noalloc
 from tests.helpers import (FIELDS, compare_state, load_oracle, random_state, small_params, smooth_state,
                            upload_from_oracle)
 
