@@ -433,6 +433,69 @@ PS3D_HD size_t thomas_smem(int nz, int threads) {
     return (size_t)((nz + kThomasChunk - 1) / kThomasChunk + 1) * threads * sizeof(double2);
 }
 
+// The (0,0) column of one instance, both parts, by one warp:
+//   p(1) = 0, p(2) = f(1) dz^2 dsqr, p(k+1) = 2p(k) - p(k-1) + f(k) dz^2 dsqr.
+// sm: room for nz complex values.  The lanes bring 256 levels at a time into
+// shared memory, lanes 0 and 1 run the recurrence there.  By a thread among
+// those of the other columns, as it was, its chunks' load latencies came on
+// top of that warp's own solve and held the whole kernel up: 128x128x64 13.2
+// us, of which a block's other warps took 7.
+template <typename R>
+__device__ __forceinline__ void zero_column(typename cpx_t<R>::type* col, long lsc, int nz, double h, typename cpx_t<R>::type* sm,
+                                            unsigned long long pk) {
+    using T = typename cpx_t<R>::type;
+    const int lane = threadIdx.x & 31;
+    for (int k0 = 0; k0 < nz; k0 += 256) {
+        T v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int k = k0 + 32 * q + lane;
+            if (k < nz) v[q] = ld_l2(&col[k * lsc], pk);
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int k = k0 + 32 * q + lane;
+            if (k < nz) sm[k] = v[q];
+        }
+    }
+    __syncwarp();
+    if (lane < 2) {
+        R* x = reinterpret_cast<R*>(sm) + lane;
+        double x0 = 0.0, x1 = 0.0, fprev = 0.0;   // p(k-2), p(k-1), f(k-1)
+        R d = x[0];
+#pragma unroll 4
+        for (int k = 0; k < nz; ++k) {
+            const R nd = k + 1 < nz ? x[2 * (k + 1)] : (R)0;
+            const double xk = k == 0 ? 0.0 : 2 * x1 - x0 + fprev * h;
+            fprev = (double)d;
+            x0 = x1; x1 = xk;
+            x[2 * k] = (R)xk;
+            d = nd;
+        }
+    }
+    __syncwarp();
+    for (int k = lane; k < nz; k += 32) st_l2(&col[k * lsc], sm[k], pk);
+}
+// The same by one thread, part by part, for any other column without a
+// wavenumber (grids whose Lx or Ly is not nx dx or ny dy may have some).
+template <typename R>
+__device__ __noinline__ void zero_part(R* col, long ls, int nz, double h, unsigned long long pk) {
+    double x0 = 0.0, x1 = 0.0, fprev = 0.0;
+    for (int k = 0; k < nz; ++k) {
+        const double d = (double)ld_l2(&col[k * ls], pk);
+        const double xk = k == 0 ? 0.0 : 2 * x1 - x0 + fprev * h;
+        fprev = d;
+        x0 = x1; x1 = xk;
+        st_l2(&col[k * ls], (R)xk, pk);
+    }
+}
+// blocks of the vertical solve after those of the columns, one warp an
+// instance; none for a slab that does not hold column (0,0)
+PS3D_HD int zero_blocks(int batch, long col0, int threads) {
+    const int wpb = threads / 32;
+    return col0 ? 0 : ((batch > 1 ? batch : 1) + wpb - 1) / wpb;
+}
+
 template <typename R, bool FULL>
 __global__ void __launch_bounds__(kThomasThreads, 4) k_thomas(const ColumnArgs a) {
     pdl_trigger();
@@ -443,6 +506,16 @@ __global__ void __launch_bounds__(kThomasThreads, 4) k_thomas(const ColumnArgs a
 #define IN(cond) (FULL || (cond))
     extern __shared__ double2 ckp[];   // [chunk][thread]: (c', d') of the level before the chunk
     const long ncols = a.ncl ? a.ncl : (long)a.nxh * a.ny;   // columns held (a column slab: ncl)
+    const int zb = zero_blocks(a.batch, a.col0, blockDim.x);
+    const int z0 = (int)gridDim.x - zb;
+    if ((int)blockIdx.x >= z0) {
+        const int w = threadIdx.x >> 5, zi = (blockIdx.x - z0) * (blockDim.x >> 5) + w;
+        using T = typename cpx_t<R>::type;
+        if (zi < a.batch)
+            zero_column<R>(reinterpret_cast<T*>(a.spec) + (long)zi * a.sM, ncols, a.nz, a.dz2dsqr,
+                           reinterpret_cast<T*>(ckp) + (size_t)w * a.nz, pk);
+        return;
+    }
     const long gid = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (gid >= 2 * ncols * a.batch) return;
     const int part = (int)(gid & 1);
@@ -532,35 +605,8 @@ __global__ void __launch_bounds__(kThomasThreads, 4) k_thomas(const ColumnArgs a
                 if (IN(kb + q < nz)) st_l2(&col[(long)(kb + q) * ls], d[q], pk);
         }
     } else {
-        // (0,0) mode: p(1) = 0, p(2) = f(1) dz^2 dsqr, p(k+1) = 2p(k) - p(k-1) + f(k) dz^2 dsqr,
-        // in chunks with the next chunk's loads in flight like the sweeps above
-        const double h = a.dz2dsqr;
-        double x0 = 0.0, x1 = 0.0, fprev = 0.0;   // p(k-2), p(k-1), f(k-1)
-        R nxt[KC];
-#pragma unroll
-        for (int q = 0; q < KC; ++q)
-            if (IN(q < nz)) nxt[q] = ld_l2(&col[(long)q * ls], pk);
-        for (int kb = 0; kb < nz; kb += KC) {
-            R d[KC];
-#pragma unroll
-            for (int q = 0; q < KC; ++q) d[q] = nxt[q];
-#pragma unroll
-            for (int q = 0; q < KC; ++q)
-                if (FULL ? (kb + KC < nz) : (kb + KC + q < nz)) nxt[q] = ld_l2(&col[(long)(kb + KC + q) * ls], pk);
-#pragma unroll
-            for (int q = 0; q < KC; ++q) {
-                const int k = kb + q;
-                if (IN(k < nz)) {
-                    const double xk = k == 0 ? 0.0 : 2 * x1 - x0 + fprev * h;
-                    fprev = (double)d[q];
-                    x0 = x1; x1 = xk;
-                    d[q] = (R)xk;
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < KC; ++q)
-                if (IN(kb + q < nz)) st_l2(&col[(long)(kb + q) * ls], d[q], pk);
-        }
+        // a column of the (0,0) mode's equation: (0,0) itself has a warp of its own
+        if (cg != 0) zero_part(col, ls, nz, a.dz2dsqr, pk);
     }
 }
 #undef IN
@@ -625,6 +671,16 @@ __global__ void __launch_bounds__(RTAB ? kThomas2RThreads : kThomasThreads, RTAB
     double* rt = ckq + (tid >> 1);   // RTAB: level jj's r at rt[jj * (T / 2)]
     const int rts = T >> 1;
     const long ncols = a.ncl ? a.ncl : (long)a.nxh * a.ny;   // columns held (a column slab: ncl)
+    const int zb = zero_blocks(a.batch, a.col0, T);
+    const int z0 = (int)gridDim.x - zb;
+    if ((int)blockIdx.x >= z0) {
+        const int w = tid >> 5, zi = (blockIdx.x - z0) * (T >> 5) + w;
+        using C = typename cpx_t<R>::type;
+        if (zi < a.batch)
+            zero_column<R>(reinterpret_cast<C*>(a.spec) + (long)zi * a.sM, ncols, nz, a.dz2dsqr,
+                           reinterpret_cast<C*>(ck2) + (size_t)w * nz, pk);
+        return;
+    }
     const long gid = blockIdx.x * (long)T + tid;
     if (gid >= 2 * ncols * a.batch) return;
     const int part = (int)(gid & 1);
@@ -641,31 +697,7 @@ __global__ void __launch_bounds__(RTAB ? kThomas2RThreads : kThomasThreads, RTAB
     const double ks = a.hkx[i] + a.hky[j];
     const double fxa = a.fxa;
     if (!(ks > 0)) {
-        // (0,0) mode: p(1) = 0, p(2) = f(1) dz^2 dsqr, p(k+1) = 2p(k) - p(k-1) + f(k) dz^2 dsqr
-        const double h = a.dz2dsqr;
-        double x0 = 0.0, x1 = 0.0, fprev = 0.0;   // p(k-2), p(k-1), f(k-1)
-        R nxt[KC];
-#pragma unroll
-        for (int q = 0; q < KC; ++q)
-            if (q < nz) nxt[q] = ld_l2(&col[(unsigned)q * ls], pk);
-        for (int kb = 0; kb < nz; kb += KC) {
-            R d[KC];
-#pragma unroll
-            for (int q = 0; q < KC; ++q) d[q] = nxt[q];
-#pragma unroll
-            for (int q = 0; q < KC; ++q)
-                if (kb + KC + q < nz) nxt[q] = ld_l2(&col[(unsigned)(kb + KC + q) * ls], pk);
-#pragma unroll
-            for (int q = 0; q < KC; ++q) {
-                const int k = kb + q;
-                if (k < nz) {
-                    const double xk = k == 0 ? 0.0 : 2 * x1 - x0 + fprev * h;
-                    fprev = (double)d[q];
-                    x0 = x1; x1 = xk;
-                    st_l2(&col[(unsigned)k * ls], (R)xk, pk);
-                }
-            }
-        }
+        if (cg != 0) zero_part(col, (long)ls, nz, a.dz2dsqr, pk);   // (0,0) itself has a warp of its own
         return;
     }
     const double bend = -ks - fxa, bmid = -ks - 2 * fxa;
@@ -1150,6 +1182,23 @@ __global__ void __launch_bounds__(kYcThreads + 256, 1) k_ycol(const YColArgs a) 
     const int inst = blockIdx.x / nxh, kx = blockIdx.x - inst * nxh;
     const int tid = threadIdx.x;
     const double fxa = a.fxa;
+    // a column without a wavenumber, one part, level k at col[2 k]
+    auto zero_col = [&](double* col) {
+        double x0 = 0.0, x1 = 0.0, fprev = 0.0;
+        for (int k0 = 0; k0 < nz; k0 += KC) {
+            double d[KC];
+#pragma unroll
+            for (int q = 0; q < KC; ++q) d[q] = k0 + q < nz ? col[2 * (k0 + q)] : 0.0;
+#pragma unroll
+            for (int q = 0; q < KC; ++q)
+                if (k0 + q < nz) {
+                    const double xk = k0 + q == 0 ? 0.0 : 2 * x1 - x0 + fprev * a.dz2dsqr;
+                    fprev = d[q];
+                    x0 = x1; x1 = xk;
+                    col[2 * (k0 + q)] = xk;
+                }
+        }
+    };
     if (tid >= NT) {
         // the pivots: r(0) = 1/b(1), r(jj) = 1/(b - cp(jj-1) a), cp = c r
         const int p = tid - NT;
@@ -1168,6 +1217,10 @@ __global__ void __launch_bounds__(kYcThreads + 256, 1) k_ycol(const YColArgs a) 
                 piv[H * ny + p] = 1.0 / (1.0 - cp * cp_jb);
             }
         }
+        __syncthreads();   // the forward transforms are done
+        // (0,0), column 0 of the transforms' order: p(1) = 0, p(2) = f(1) dz^2 dsqr,
+        // p(k+1) = 2p(k) - p(k-1) + f(k) dz^2 dsqr
+        if (kx == 0 && p < 2) zero_col(reinterpret_cast<double*>(buf) + p);
         __syncthreads();
         return;
     }
@@ -1214,21 +1267,7 @@ __global__ void __launch_bounds__(kYcThreads + 256, 1) k_ycol(const YColArgs a) 
         double* col = reinterpret_cast<double*>(buf + (size_t)p * ld) + (c & 1);   // level k at col[2 k]
         const double* pv = piv + p;                                              // pivot level jj at pv[jj ny]
         if (!(pv[0] != 0.0)) {
-            // (0,0): p(1) = 0, p(2) = f(1) dz^2 dsqr, p(k+1) = 2p(k) - p(k-1) + f(k) dz^2 dsqr
-            double x0 = 0.0, x1 = 0.0, fprev = 0.0;
-            for (int k0 = 0; k0 < nz; k0 += KC) {
-                double d[KC];
-#pragma unroll
-                for (int q = 0; q < KC; ++q) d[q] = k0 + q < nz ? col[2 * (k0 + q)] : 0.0;
-#pragma unroll
-                for (int q = 0; q < KC; ++q)
-                    if (k0 + q < nz) {
-                        const double xk = k0 + q == 0 ? 0.0 : 2 * x1 - x0 + fprev * a.dz2dsqr;
-                        fprev = d[q];
-                        x0 = x1; x1 = xk;
-                        col[2 * (k0 + q)] = xk;
-                    }
-            }
+            if (kx != 0 || p != 0) zero_col(col);   // (0,0) itself: the pivots' threads
             continue;
         }
         double* bot = col + 2 * (nz - 1);   // bottom chain: level nz-1-jj at bot[-2 jj]
@@ -1280,6 +1319,7 @@ __global__ void __launch_bounds__(kYcThreads + 256, 1) k_ycol(const YColArgs a) 
             }
         }
     }
+    __syncthreads();   // column (0,0)
     fft_batch<true, double, MAXR, true, NT>(buf, ld, nz, a.py, +1, ty.tw, a.nslots);
     for (int t = tid; t < total; t += NT) {
         const int k = (int)fdiv(t, a.fd_ny), j = t - k * ny;
@@ -2460,17 +2500,29 @@ cudaError_t launch_thomas(const ColumnArgs& a0, bool fp32, cudaStream_t s) {
     a.fd_nxh = make_fastdiv(a.nxh);
     // the two-ended form with two threads per column where 4 blocks of 128
     // fit an SM, else the one-ended form with as many threads per block as
-    // its checkpoints allow; PS3D_THOMAS_FORM=0|2|3 pins one (3: the
-    // two-ended form with its pivot table); PS3D_THOMAS_FULL=0 keeps the
-    // bounds-tested instantiation of the two-ended form on every grid
+    // its checkpoints allow.  Of the two-ended ones that with its pivot table
+    // where the grid is resident at once, FP32 also where eight of its blocks
+    // fit an SM (without the table and with it: 256x256x64 FP64 15.0 and 13.4
+    // us, 256x256x128 25.2 and 23.5, FP32 23.4 and 22.2, 512x512x128 FP32
+    // 92.6 and 85.9; but 512x256x128 FP64 58 and 69, where the table's shared
+    // memory is taken from the L1 that the way back reads, and 256x256x192
+    // FP32 31.5 and 38.7, where six blocks fit).  PS3D_THOMAS_FORM=0|2|3 pins
+    // one (3: with the table); PS3D_THOMAS_FULL=0 keeps the bounds-tested
+    // instantiation of the two-ended form on every grid
     const char* pin = std::getenv("PS3D_THOMAS_FORM");
     const char* fe = std::getenv("PS3D_THOMAS_FULL");
-    const int form = pin ? pin[0] - '0' : (thomas2_smem(a.nz, kThomasThreads) <= 56 * 1024 ? 2 : 0);
+    a.batch = std::max(1, a.batch);
+    const long n2 = 2 * ncols * a.batch;
+    auto table_form = [&] {
+        const long res = std::min<long>(8, 228 * 1024 / (thomas2r_smem(a.nz, kThomas2RThreads) + 1024));   // blocks an SM
+        const long blocks = (n2 + kThomas2RThreads - 1) / kThomas2RThreads + zero_blocks(a.batch, a.col0, kThomas2RThreads);
+        return blocks <= 148 * res || (fp32 && res == 8);
+    };
+    const int form = pin ? pin[0] - '0' : (thomas2_smem(a.nz, kThomasThreads) > 56 * 1024 ? 0 : table_form() ? 3 : 2);
     const bool off32 = (long)a.nz * 2 * ncols < (1L << 32);   // 32-bit level offsets
     const bool full = a.nz % (2 * kThomasChunk) == 0 && !(fe && fe[0] == '0');
-    const long n2 = 2 * ncols * std::max(1, a.batch);
     if (form == 3 && off32 && thomas2r_smem(a.nz, kThomas2RThreads) <= 227 * 1024 - 64) {
-        const dim3 g((unsigned)((n2 + kThomas2RThreads - 1) / kThomas2RThreads)), b(kThomas2RThreads);
+        const dim3 g((unsigned)((n2 + kThomas2RThreads - 1) / kThomas2RThreads) + zero_blocks(a.batch, a.col0, kThomas2RThreads)), b(kThomas2RThreads);
         const size_t sm = thomas2r_smem(a.nz, kThomas2RThreads);
         if (full) return fp32 ? launch_pdl(k_thomas2<float, true, true>, g, b, sm, s, a)
                               : launch_pdl(k_thomas2<double, true, true>, g, b, sm, s, a);
@@ -2478,7 +2530,7 @@ cudaError_t launch_thomas(const ColumnArgs& a0, bool fp32, cudaStream_t s) {
                     : launch_pdl(k_thomas2<double, false, true>, g, b, sm, s, a);
     }
     if (form == 2 && off32 && thomas2_smem(a.nz, kThomasThreads) <= 227 * 1024 - 64) {
-        const dim3 g((unsigned)((n2 + kThomasThreads - 1) / kThomasThreads)), b(kThomasThreads);
+        const dim3 g((unsigned)((n2 + kThomasThreads - 1) / kThomasThreads) + zero_blocks(a.batch, a.col0, kThomasThreads)), b(kThomasThreads);
         const size_t sm = thomas2_smem(a.nz, kThomasThreads);
         if (full) return fp32 ? launch_pdl(k_thomas2<float, true, false>, g, b, sm, s, a)
                               : launch_pdl(k_thomas2<double, true, false>, g, b, sm, s, a);
@@ -2487,8 +2539,7 @@ cudaError_t launch_thomas(const ColumnArgs& a0, bool fp32, cudaStream_t s) {
     }
     const int nt = thomas_threads(a.nz);
     if (nt == 0 || ncols < 1) return cudaErrorInvalidValue;
-    const long nthreads = 2 * ncols * std::max(1, a.batch);
-    const int blocks = (int)((nthreads + nt - 1) / nt);
+    const int blocks = (int)((n2 + nt - 1) / nt) + zero_blocks(a.batch, a.col0, nt);
     const size_t sm = thomas_smem(a.nz, nt);
     const dim3 g(blocks), b(nt);
     if (a.nz % kThomasChunk == 0) {
