@@ -24,32 +24,74 @@
 
 namespace ps3d {
 
-__global__ void k_project(const ProjArgs a) {
-    const long M = (long)a.nxh * a.ny * a.nz;
-    const Phys P{a.f0, a.N0, a.dsqr, a.dz};
-    for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < M; t += (long)gridDim.x * blockDim.x) {
-        const int i = a.layout ? (int)((t / a.ny) % a.nxh) : (int)(t % a.nxh);
-        const int j = a.layout ? (int)(t % a.ny) : (int)((t / a.nxh) % a.ny);
-        const int k = (int)(t / ((long)a.nxh * a.ny));
-        Ax x{a.ax.kx[i], a.ax.hkx[i], a.ax.ex[i], ld(a.ax.px + i), a.dx};
-        Ax y{a.ax.ky[j], a.ax.hky[j], a.ax.ey[j], ld(a.ax.py + j), a.dy};
-        cz_t q[4], p[4];
+// The geostrophic vectors (s = 0) of vec_qp_vbc and vec_qp_discrete, split by
+// what they depend on: at s = 0 the horizontal components belong to the column,
+// the buoyancy one to the level, w has none, and a point adds the
+// normalisation.  A thread keeps a column and walks up to kProjLevels levels,
+// their tables in shared memory.  Formed point by point, ten FP64 divisions
+// and a square root each, the kernel was bound by them at 131 us for
+// 256x256x64, where its four fields in and out take 42; it now takes 57 us.
+constexpr int kProjLevels = 16;
+constexpr int kProjThreads = 128;
+
+__global__ void __launch_bounds__(kProjThreads) k_project(const ProjArgs a, int kchunk) {
+    __shared__ double sN2[kProjLevels], sm2[kProjLevels];
+    __shared__ cz_t sqb[kProjLevels];
+    const int k0 = blockIdx.y * kchunk, nk = min(kchunk, a.nz - k0);
+    const double N02 = a.N0 * a.N0;
+    if ((int)threadIdx.x < nk) {
+        const int k = k0 + threadIdx.x;
+        double N2_hat, m2;
+        cz_t qb = Cz(0, 0);
         if (a.rigid) {
-            vec_qp_vbc(x, y, a.ax.kz[k], a.ax.sz[k], a.ax.cz[k], 0.0, P, q, p);
+            const double sarg = a.ax.sz[k], carg = a.ax.cz[k], kz = a.ax.kz[k];
+            N2_hat = N02 * (carg * carg);
+            m2 = 4 * (sarg * sarg) / (a.dz * a.dz);
+            if (kz * kz > 0.0) qb = Cz(-(2 * sarg / a.dz * carg * N02 / N2_hat), 0.0);
         } else {
-            Ax z{a.ax.kz[k], a.ax.hkz[k], a.ax.ez[k], ld(a.ax.pz + k), a.dz};
-            vec_qp_discrete(x, y, z, 0.0, P, q, p);
+            const Ax z{a.ax.kz[k], a.ax.hkz[k], a.ax.ez[k], ld(a.ax.pz + k), a.dz};
+            N2_hat = N02 * z.ep;
+            m2 = z.hk;
+            if (z.k * z.k > 0.0) qb = Cz(0, 1) * hat_em(z) * hat_kp(z) * N02 / N2_hat;
         }
+        sN2[threadIdx.x] = N2_hat;
+        sm2[threadIdx.x] = m2;
+        sqb[threadIdx.x] = qb;
+    }
+    __syncthreads();
+    const unsigned ncol = (unsigned)a.nxh * a.ny, c = blockIdx.x * kProjThreads + threadIdx.x;
+    if (c >= ncol) return;
+    const int i = (int)(a.layout ? c / (unsigned)a.ny : c % (unsigned)a.nxh);
+    const int j = (int)(a.layout ? c - (unsigned)i * a.ny : c / (unsigned)a.nxh);
+    const Ax x{a.ax.kx[i], a.ax.hkx[i], a.ax.ex[i], ld(a.ax.px + i), a.dx};
+    const Ax y{a.ax.ky[j], a.ax.hky[j], a.ax.ey[j], ld(a.ax.py + j), a.dy};
+    const cz_t IM = Cz(0, 1);
+    const double f2_hat = (a.f0 * a.f0) * x.ep * y.ep, k2 = x.hk + y.hk;
+    const bool wave = x.k * x.k + y.k * y.k > 0.0;
+    cz_t qxc = Cz(0, 0), qyc = Cz(0, 0);
+    if (wave) {
+        qxc = -(IM * a.f0 * hat_ep(x) * hat_em(y) * hat_kp(y)) / f2_hat;
+        qyc = (IM * a.f0 * hat_em(x) * hat_ep(y) * hat_kp(x)) / f2_hat;
+    }
+    long t = (long)k0 * ncol + c;
+#pragma unroll 2
+    for (int kk = 0; kk < nk; ++kk, t += ncol) {
         const cz_t US = ld(a.US + t), VS = ld(a.VS + t), WS = ld(a.WS + t), BS = ld(a.BS + t);
-        const cz_t g0 = p[0] * US + p[1] * VS + p[2] * WS + p[3] * BS;
+        const double N2_hat = sN2[kk], m2 = sm2[kk];
+        const bool zero = f2_hat == 0.0 || N2_hat == 0.0;
+        const cz_t qx = zero ? Cz(0, 0) : qxc, qy = zero ? Cz(0, 0) : qyc, qz = Cz(0, 0);
+        const cz_t qb = zero || !wave ? Cz(0, 0) : sqb[kk];
+        const double dd = k2 * N2_hat + f2_hat * m2;
+        const double pc = dd > 0.0 ? f2_hat * N2_hat / dd : 0.0;
+        const cz_t g0 = pc * conjg(qx) * US + pc * conjg(qy) * VS + pc * conjg(qz) * a.dsqr * WS + pc * conjg(qb) / N02 * BS;
         if (a.mode == PS3D_PROJ_EXCHANGE) {
             const cz_t d = ld(a.g0base + t) - g0;
-            st(a.US + t, US + d * q[0]); st(a.VS + t, VS + d * q[1]);
-            st(a.WS + t, WS + d * q[2]); st(a.BS + t, BS + d * q[3]);
+            st(a.US + t, US + d * qx); st(a.VS + t, VS + d * qy);
+            st(a.WS + t, WS + d * qz); st(a.BS + t, BS + d * qb);
         } else {
             if (a.mode == PS3D_PROJ_BASE_POINT) st(a.g0base + t, g0);
-            st(a.US + t, g0 * q[0]); st(a.VS + t, g0 * q[1]);
-            st(a.WS + t, g0 * q[2]); st(a.BS + t, g0 * q[3]);
+            st(a.US + t, g0 * qx); st(a.VS + t, g0 * qy);
+            st(a.WS + t, g0 * qz); st(a.BS + t, g0 * qb);
         }
     }
 }
@@ -130,9 +172,10 @@ __global__ void __launch_bounds__(kVmThreads) k_vert_mode(const double2* __restr
 }
 
 cudaError_t launch_project(const ProjArgs& a, cudaStream_t s) {
-    const long M = (long)a.nxh * a.ny * a.nz;
-    const int blocks = (int)std::min<long>((M + 255) / 256, 148L * 16);
-    k_project<<<blocks, 256, 0, s>>>(a);
+    const long ncol = (long)a.nxh * a.ny, bx = (ncol + kProjThreads - 1) / kProjThreads;
+    int kc = kProjLevels;   // fewer levels a thread where the blocks would not fill the GPU
+    while (kc > 2 && bx * ((a.nz + kc - 1) / kc) < 148 * 4) kc /= 2;
+    k_project<<<dim3((unsigned)bx, (unsigned)((a.nz + kc - 1) / kc)), kProjThreads, 0, s>>>(a, kc);
     return cudaGetLastError();
 }
 

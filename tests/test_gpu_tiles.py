@@ -188,3 +188,17 @@ def test_noalloc_projection_shapes(rigid):
             # a velocity carries p's rounding times dt over its grid distance
             tol = TOL_KERNEL + (8 * np.finfo(float).eps * p.dt / d * pn / np.linalg.norm(want) if d else 0.0)
             assert np.linalg.norm(got[k] - want) <= tol * np.linalg.norm(want), (n, k)
+
+
+@pytest.mark.parametrize("rigid", [True, False])
+@pytest.mark.parametrize("n", [(18, 10, 6), (36, 30, 20), (128, 128, 70), (256, 128, 36)])
+def test_projection_columns(n, rigid):
+    """The eigenvector projection by columns: fewer columns than a block, a
+    last block that is not full, chunks of 2, 4 and 8 levels with a remainder."""
+    nz = n[2] if rigid else {6: 6, 20: 20, 70: 72, 36: 36}[n[2]]
+    p = small_params(n[0], n[1], nz, rigid=rigid, Lz=1000.0 * nz / 16)
+    o, m = _pair(p, smooth_state(p, seed=47))
+    o.project(abi.PS3D_PROJ_NORMAL_MODE)
+    m.project(abi.PS3D_PROJ_NORMAL_MODE)
+    err = compare_state(m, o, names=FIELDS)
+    assert max(err.values()) < TOL_KERNEL, err
