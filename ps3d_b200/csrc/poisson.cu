@@ -34,6 +34,11 @@ constexpr int kPlaneThreads = 256;
 // blocks per SM the plane kernels are built for: the radix-16 instantiation
 // needs ~128 FP64 registers, the radix-8 one fits in 80
 template <int MAXR> constexpr int plane_min_blocks() { return MAXR >= 16 ? 2 : 3; }
+// Rows passes: four blocks where they fit 64 registers (forward transforms
+// 256x256x128 FP64 92.2 -> 89.1 us, 512x256x64 95.1 -> 92.9, 128x128x64 22.8 ->
+// 21.0; inverse 320x200x64 60.1 -> 57.2); the forward loads with the pressure's
+// would spill.
+template <int MAXR, int MODE> constexpr int rows_blocks() { return MAXR <= 8 && MODE != 2 ? 4 : plane_min_blocks<MAXR>(); }
 template <typename R, int MAXR> constexpr int lines_min_blocks() { return MAXR >= 16 ? 2 : 4; }
 
 // the L2 policies of a kernel (PlaneArgs/ColumnArgs::l2hint): the spectra
@@ -109,7 +114,7 @@ __device__ __forceinline__ double2 plane_source_pair(const PlaneArgs& a, const d
 // index arithmetic; forward transforms, before and after: 256x256x128 FP64 99.4
 // and 92.5 us, 512x256x64 94.4 and 86.6 us mixed, 128x128x64 25.5 and 20.0 us
 // mixed.  LB is chosen against registers: two rows in flight in FP64 (four
-// spill the 80 registers of three blocks, 117 us), one with the pressure's
+// spill, 117 us), one with the pressure's
 // seven further loads (two cost the FP32 register pass blocks: 108.9 against
 // 86.6 us at 512x256x64), two where a thread walks only 8 rows (nx = 128).
 template <int MODE, int LB, class Store>
@@ -1579,7 +1584,7 @@ __global__ void __launch_bounds__(kZRegThreads, 4) k_zsolve_reg(const ColumnArgs
 // flight.
 // ---------------------------------------------------------------------------
 template <typename R, int MAXR, int MODE>
-__global__ void __launch_bounds__(kPlaneThreads, plane_min_blocks<MAXR>()) k_rows_fwd(const PlaneArgs a) {
+__global__ void __launch_bounds__(kPlaneThreads, rows_blocks<MAXR, MODE>()) k_rows_fwd(const PlaneArgs a) {
     pdl_trigger();
     pdl_wait();   // inputs written by the preceding kernels
     const unsigned long long pfield = pol_field(a.l2hint), pkeep = pol_keep(a.l2hint);
@@ -2019,8 +2024,13 @@ __global__ void __launch_bounds__(RowReg<N1, N2, R>::NT) k_rows_fwd_reg(const Pl
 // transforms E' (even ky) and O' (odd ky) of [k][kx][half][j], rows j and
 // j+ny/2 of the inverse y transform are E'_j + w_ny^-j O'_j and
 // E'_j - w_ny^-j O'_j.
+// registers: a block an SM as the bound lets the compiler hold all of a
+// batch's loads, to the good where a row has 8 threads (128x128x64 FP32 16.1 ->
+// 14.5 us for the inverse, 256x256x128 FP32 41.4 -> 39.2), not where it has 16
+// (512x256x64 FP32 43.8 -> 51.6) nor in FP64 with 16 elements a thread (55.8 ->
+// 57.7 at 256x256x128)
 template <typename R, int N1, int N2, bool YS>
-__global__ void __launch_bounds__(RowReg<N1, N2, R>::NT) k_rows_inv_reg(const PlaneArgs a) {
+__global__ void __launch_bounds__(RowReg<N1, N2, R>::NT, N1 == 8 || (N2 == 8 && sizeof(R) == 4) ? 1 : 0) k_rows_inv_reg(const PlaneArgs a) {
     pdl_trigger();
     pdl_wait();   // inputs written by the preceding kernels
     const unsigned long long plast = pol_last(a.l2hint);
@@ -2133,7 +2143,7 @@ __global__ void __launch_bounds__(RowReg<N1, N2, R>::NT) k_rows_inv_reg(const Pl
 }
 
 template <typename R, int MAXR>
-__global__ void __launch_bounds__(kPlaneThreads, plane_min_blocks<MAXR>()) k_rows_inv(const PlaneArgs a) {
+__global__ void __launch_bounds__(kPlaneThreads, rows_blocks<MAXR, 0>()) k_rows_inv(const PlaneArgs a) {
     pdl_trigger();
     pdl_wait();   // inputs written by the preceding kernels
     const unsigned long long plast = pol_last(a.l2hint);
