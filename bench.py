@@ -53,9 +53,9 @@ def set_grid(nx, ny, nz):
 # traffic already streams far beyond L2, so it scales with the grid points;
 # the ncu commands that produced these figures are kept with the profiles.
 MEASURED_TRAFFIC_PER_POINT = {
-    "fp64": {"step": 165.8},
-    "mixed": {"step": 128.4},
-    "mixed_refined": {"step": 128.4},   # the same step kernel
+    "fp64": {"step": 164.1},
+    "mixed": {"step": 127.2},
+    "mixed_refined": {"step": 127.2},   # the same step kernel
 }
 
 # algorithmic HBM bytes per grid point per launch.  The step kernel reads
