@@ -722,12 +722,17 @@ bool ycol_enabled(int nz, int ny) {
     return !(e && e[0] == '0') && ycol_fits(nz, ny);
 }
 bool Ctx::ycol_allowed() const { return !mixed && rigid && !split_solve && ycol_enabled(nz, ny); }
-// Untuned (tiny) grids: fused where every kx has an SM of its own.  Per step,
-// apart and fused: 32x32x16 23.9 and 19.1 us, 48x40x24 28.7 and 21.9 us.
-// Tuned grids take the faster of the two: 96x80x50 51.3 and 43.6 us,
-// 128x128x32 50.9 and 45.7 us, 64x64x32 28.7 and 27.3 us, but 64x128x64 53.4
-// and 54.0 us (a block's 131 KB of spectra leave 33 of 148 SMs at work).
-bool Ctx::ycol_default() const { return (long)nxh * batch <= 148; }
+// Untuned grids: fused where every kx has an SM of its own.  Per step, apart
+// and fused: 32x32x16 23.6 and 18.9 us, 48x40x24 29.1 and 22.5 us, 64x64x32
+// 29.2 and 27.0 us.  Tuned grids take the faster of the two: 96x80x50 49.6 and
+// 44.6 us, 128x128x32 51.1 and 45.2 us, but 64x128x64 53.4 and 54.0 us (a
+// block's 131 KB of spectra leave 33 of 148 SMs at work).
+// The grid alone decides, not the batch: the two forms round differently, and
+// a request served in a group gets the bits it gets alone.  That costs some
+// batches a little (apart and fused: 4 x 64x64x32 51.2 and 47.7 us, 16 x
+// 64x64x32 142.6 and 150.7 us, 8 x 96x80x50 222 and 202 us, 16 x 128x64x32 227
+// and 247 us).
+bool Ctx::ycol_default() const { return nxh <= 148; }
 
 int Ctx::autotune() {
     std::lock_guard<std::mutex> tune_lock(g_tune_mu);
