@@ -766,30 +766,30 @@ int Ctx::autotune() {
         }
         return false;
     };
-    // PS3D_TUNE pins a configuration in the cache's format, e.g.
-    // "im1,C1,rc8,tj16,ly8,pol2,kc8" (reproducible profiling, no timing runs)
-    auto parse = [](const char* str, int* v) {
-        v[7] = 0;   // optional: the fused y transforms and vertical solve
-        return std::sscanf(str, "im%d,C%d,rc%d,tj%d,ly%d,pol%d,kc%d,yf%d", &v[0], &v[1], &v[2], &v[3], &v[4], &v[5],
-                           &v[6], &v[7]) >= 7;
+    // a configuration in the cache's format: true if it was one of this grid's
+    // shapes, now taken.  The suffix yf1 (the fused y transforms and vertical
+    // solve) counts with the rows passes alone: the cluster kernels transform
+    // along y themselves.
+    auto take = [&](const char* str) -> bool {
+        int v[8] = {};
+        if (std::sscanf(str, "im%d,C%d,rc%d,tj%d,ly%d,pol%d,kc%d,yf%d", &v[0], &v[1], &v[2], &v[3], &v[4], &v[5], &v[6],
+                        &v[7]) < 7 ||
+            !apply(v[0], v[1], v[2], v[3], v[4], v[5], v[6]))
+            return false;
+        yfused = v[7] && ycol_allowed() && pa.impl >= 1;
+        return true;
     };
+    // PS3D_TUNE pins a configuration, e.g. "im1,C1,rc8,tj16,ly8,pol2,kc8"
+    // (reproducible profiling, no timing runs)
     if (const char* pin = std::getenv("PS3D_TUNE")) {
-        int v[8];
-        if (parse(pin, v) && apply(v[0], v[1], v[2], v[3], v[4], v[5], v[6])) {
-            yfused = v[7] && ycol_allowed();
-            tuned = std::string("pinned:") + pin;
-            return PS3D_OK;
-        }
-        return PS3D_ERR_BADPARAM;
+        if (!take(pin)) return PS3D_ERR_BADPARAM;
+        tuned = std::string("pinned:") + pin;
+        return PS3D_OK;
     }
     auto it = tune_cache().find(key);
-    if (it != tune_cache().end()) {
-        int v[8];
-        if (parse(it->second.c_str(), v) && apply(v[0], v[1], v[2], v[3], v[4], v[5], v[6])) {
-            yfused = v[7] && ycol_allowed();
-            tuned = std::string("cached:") + it->second;
-            return PS3D_OK;
-        }
+    if (it != tune_cache().end() && take(it->second.c_str())) {
+        tuned = std::string("cached:") + it->second;
+        return PS3D_OK;
     }
     if (!tune_timing) return PS3D_OK;   // the defaults chosen at init
     cudaEvent_t e0, e1;

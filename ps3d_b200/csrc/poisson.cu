@@ -1333,7 +1333,8 @@ __global__ void __launch_bounds__(kYcThreads + 256, 1) k_ycol(const YColArgs a) 
 }
 
 cudaError_t launch_ycol(const PlaneArgs& p, const ColumnArgs& c, cudaStream_t s) {
-    if (!ycol_fits(c.nz, c.ny)) return cudaErrorInvalidValue;
+    // the rows passes' layout [k][kx][ky], not yet transformed along y
+    if (p.impl < 1 || !p.yfused || !ycol_fits(c.nz, c.ny)) return cudaErrorInvalidValue;
     YColArgs a{};
     a.nz = c.nz; a.ny = c.ny; a.nxh = c.nxh;
     a.spec = reinterpret_cast<double2*>(c.spec); a.sM = c.sM;

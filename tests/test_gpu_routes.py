@@ -4,9 +4,13 @@ import numpy as np
 import pytest
 
 from ps3d_b200 import abi
+from ps3d_b200.model import Model
 from ps3d_b200.serve import Server, request
+from oracle.binding import Oracle
+from tests.helpers import FIELDS, compare_state, load_oracle, random_state, small_params
 
 pytestmark = pytest.mark.gpu
+TOL_KERNEL = 1e-12   # one FP64 pressure solve
 
 
 @pytest.mark.parametrize("n", [(128, 16, 8), (96, 20, 10)])
@@ -32,3 +36,22 @@ def test_batched_requests_match_alone_on_wide_grids(n, monkeypatch):
         assert a.status == g.status == 0 and g.iters == a.iters and g.norm == a.norm
         for k in ("u", "v", "w", "b"):
             assert np.array_equal(g.fields[k], a.fields[k]), k
+
+
+@pytest.mark.parametrize("pin,fused", [("im0,C1,rc4,tj8,ly8,pol1,kc4", 0), ("im1,C1,rc8,tj16,ly16,pol1,kc4", 1),
+                                       ("im2,C1,rc8,tj8,ly16,pol2,kc4", 1)])
+def test_pinned_fused_solve(pin, fused, monkeypatch):
+    """A pin's suffix yf1 takes the fused y transforms and vertical solve where
+    the pinned plane form feeds them, and is without effect on the cluster
+    form, which transforms along y itself."""
+    monkeypatch.setenv("PS3D_TUNE", pin + ",yf1")
+    p = small_params(32, 32, 10, rigid=True)
+    f = random_state(p, seed=51)
+    o, m = Oracle(p), Model(p)
+    load_oracle(o, f)
+    m.upload(**{k: f[k] for k in FIELDS})
+    o.pressure_solver()
+    m.pressure_solver()
+    assert f"yfused={fused}" in m.describe() and "tuned=pinned" in m.describe()
+    err = compare_state(m, o)
+    assert max(err.values()) < TOL_KERNEL, err
