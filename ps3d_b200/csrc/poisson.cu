@@ -23,6 +23,7 @@
 #include <cstdlib>
 #include "engine.h"
 #include "async.cuh"
+#include "divide.cuh"
 #include "fft.cuh"
 
 namespace cg = cooperative_groups;
@@ -410,27 +411,8 @@ __global__ void __launch_bounds__(kPlaneThreads, plane_min_blocks<MAXR>()) k_pla
 // chunk with x.  The pivots are formed from ksqr on the fly (rcp_newton):
 // no factor table and no d' array in HBM.
 // ---------------------------------------------------------------------------
-// The FP64 reciprocal of a pivot by Newton-Raphson from the hardware
-// approximation (PTX rcp.approx.ftz.f64): each iteration y += y (1 - x y)
-// squares the relative error, two take it far below the FP64 rounding unit,
-// and a third, with the residual 1 - x y formed exactly by an FMA, rounds
-// the result correctly (Markstein, "Computation of elementary functions on
-// the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990); on a
-// B200 it agreed bit for bit with the correctly rounded 1.0 / x on 2^30
-// random inputs over 81 binades, in fewer instructions.  The pivots are
-// normal numbers bounded away from zero (the matrix is strictly diagonally
-// dominant), so the flush-to-zero approximation never sees a subnormal.
-__device__ __forceinline__ double rcp_newton(double x) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    double e = fma(-x, y, 1.0);
-    y = fma(y, e, y);
-    e = fma(-x, y, 1.0);
-    y = fma(y, e, y);
-    e = fma(-x, y, 1.0);
-    return fma(y, e, y);
-}
-
+// The pivots are normal numbers bounded away from zero (the matrix is strictly
+// diagonally dominant), as rcp_newton wants them.
 constexpr int kThomasChunk = 8;
 constexpr int kThomasThreads = 128;
 
@@ -1385,38 +1367,6 @@ cudaError_t launch_colsolve(const PlaneArgs& p, const ColumnArgs& c, cudaStream_
 // ---------------------------------------------------------------------------
 constexpr int kZLines = 32;
 
-// the spectral value times -1/ksqr (pressure_solver.f90:59-69), zero where
-// ksqr is.  One reciprocal for both parts; FP32 takes it to the quotients that
-// an FP64 division of each part rounds to: with r = 1/ks rounded, q = a r is
-// within 1.5 units of the last place, one step q += r (a - q ks) brings it
-// within one, and the second, whose residual is exact, rounds it correctly
-// (Markstein 1990, as above).  Zeros, infinities and NaNs take the first
-// product, and a ksqr so extreme that a step could leave the normal numbers is
-// divided by.  Equal to the division on 2^33 random operands; with two
-// divisions an element FP32 took longer than FP64: 512x256x64 47.2 us, now
-// 33.4.
-template <typename R>
-__device__ __forceinline__ cpx<R> z_divide(cpx<R> v, double ks) {
-    if (!(ks > 0.0)) return mk<R>((R)0, (R)0);
-    if constexpr (sizeof(R) == 8) {
-        const double r = -1.0 / ks;
-        return mk<R>(v.x * r, v.y * r);
-    } else {
-        if (!(ks > 1e-200 && ks < 1e200)) return mk<R>((R)(-(double)v.x / ks), (R)(-(double)v.y / ks));
-        const double r = rcp_newton(ks);
-        auto quot = [&](float f) {
-            const double d = -(double)f;
-            double q = d * r;
-            if (fabsf(f) > 0.0f && fabsf(f) <= 3.402823466e+38f) {
-                q = fma(fma(-q, ks, d), r, q);
-                q = fma(fma(-q, ks, d), r, q);
-            }
-            return (float)q;
-        };
-        return mk<R>(quot(v.x), quot(v.y));
-    }
-}
-
 // Columns staged in shared memory, any length that factors: a lane keeps one
 // column, so no index is divided (256x256x96 FP64 92 -> 59 us, FP32 90 -> 51).
 template <typename R>
@@ -1464,7 +1414,7 @@ __global__ void __launch_bounds__(256, 2) k_zsolve(const ColumnArgs a) {
         if (on)
             for (int p = kw; p < nz; p += nw) {
                 T v = cscale(buf[p * ld + l], sc);
-                if (a.op == 0) v = z_divide<R>(v, k2 + a.hkz[tz.ipos[p]]);
+                if (a.op == 0) v = divide_neg<R>(v, k2 + a.hkz[tz.ipos[p]]);
                 buf[p * ld + l] = v;
             }
         if (a.op == 0) fft_batch<true, R, 16, true>(buf, ld, nl, a.pz, +1, tz.tw, kZLines);
@@ -1485,10 +1435,10 @@ __global__ void __launch_bounds__(256, 2) k_zsolve(const ColumnArgs a) {
 // Two shared-memory round trips an element against the staged kernel's six
 // (bound by them and by its latency at three blocks an SM).  The butterflies
 // and twiddles are the staged kernel's for the plan {16, N1}, in its order:
-// the same bits in FP32 (in FP64 too but for the shared reciprocal).
+// the same bits in FP32.
 // Bound by its FP64 arithmetic and two block barriers at four blocks an SM:
-// 512x256x128 80 us FP64 (270 MB, 52 % of the copy bandwidth) and 64 us FP32,
-// where the staged kernel with divided indices took 206 and 165 us.
+// 512x256x128 78 us FP64 (270 MB, 54 % of the copy bandwidth) and 56 us FP32,
+// where the staged kernel with divided indices took 224 and 199 us.
 constexpr int kZRegThreads = 128;
 
 template <typename R, int N1>
@@ -1533,7 +1483,7 @@ __global__ void __launch_bounds__(kZRegThreads, 4) k_zsolve_reg(const ColumnArgs
             const long c = (on ? c0 : 0) + a.col0;   // global column: its wavenumbers
             const double k2s = a.hkx[a.layout ? c / a.ny : c % a.nxh] + a.hky[a.layout ? c % a.ny : c / a.nxh];
 #pragma unroll
-            for (int k2 = 0; k2 < N2; ++k2) v[k2] = z_divide<R>(cscale(v[k2], sc), k2s + __ldg(a.hkz + t + N1 * k2));
+            for (int k2 = 0; k2 < N2; ++k2) v[k2] = divide_neg<R>(cscale(v[k2], sc), k2s + __ldg(a.hkz + t + N1 * k2));
         } else {
             if (on) {
 #pragma unroll
