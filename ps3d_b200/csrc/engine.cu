@@ -796,13 +796,12 @@ int Ctx::autotune() {
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
     // the best of five runs, or of three times three short ones (launches start
-    // on a grid of about 2 us, coarser than the differences between small kernels)
-    auto timeit = [&](auto&& fn) -> float {
-        float best = 1e30f;
-        if (fn() != PS3D_OK) return best;
-        if (cudaStreamSynchronize(stream) != cudaSuccess) { cudaGetLastError(); return best; }
-        int reps = 1;
-        for (int r = 0; r < (reps > 1 ? 4 : 6); ++r) {
+    // on a grid of about 2 us, coarser than the differences between small
+    // kernels).  A candidate whose first run, or first warm one, is far behind
+    // the best so far gets no further ones: of the hundred or so candidates of a
+    // grid few are near it, and a context's creation is mostly these runs.
+    auto timeit = [&](float sofar, auto&& fn) -> float {
+        auto once = [&](int reps) -> float {   // ms a run, 1e30 for a failed one
             cudaEventRecord(e0, stream);
             for (int q = 0; q < reps; ++q)
                 if (fn() != PS3D_OK) return 1e30f;
@@ -810,23 +809,32 @@ int Ctx::autotune() {
             if (cudaEventSynchronize(e1) != cudaSuccess) { cudaGetLastError(); return 1e30f; }
             float ms = 0.f;
             cudaEventElapsedTime(&ms, e0, e1);
-            if (r == 0) reps = ms < 0.5f ? 3 : 1;
-            else best = std::min(best, ms / reps);
-        }
+            return ms / reps;
+        };
+        float best = once(1);
+        if (best > 2.f * sofar + 0.02f) return best;
+        best = once(1);
+        if (best > 1.2f * sofar + 0.004f) return best;
+        const int reps = best < 0.5f ? 3 : 1;
+        if (reps > 1) best = 1e30f;   // measured too coarsely
+        for (int r = reps > 1 ? 0 : 1; r < (reps > 1 ? 3 : 5); ++r) best = std::min(best, once(reps));
         return best;
     };
-    // plane kernels
+    // plane kernels, the rows passes first: they are the faster ones at every
+    // size measured
     float best = 1e30f;
     PlaneArgs bestpa = pa;
     int bestpol = 0;
-    for (const PlaneArgs& cand : plane_candidates(nx, ny, f32 ? sizeof(float2) : sizeof(double2), pa)) {
+    std::vector<PlaneArgs> cands = plane_candidates(nx, ny, f32 ? sizeof(float2) : sizeof(double2), pa);
+    std::stable_partition(cands.begin(), cands.end(), [](const PlaneArgs& c) { return c.impl == 1; });
+    for (const PlaneArgs& cand : cands) {
         for (int pol = 0; pol < 3; ++pol) {
             PlaneArgs a = cand;
             plans_of(pol, a);
             a.batch = batch;
             if (plane_force >= 0 && a.impl != plane_force) continue;
             if (a.impl == 0 && (plane_max_clusters(a, f32, true) < 1 || plane_max_clusters(a, f32, false) < 1)) continue;
-            const float t = timeit([&]() -> int {
+            const float t = timeit(best, [&]() -> int {
                 PlaneArgs f = a;
                 f.mode = 0; f.u = field(0); f.v = field(1); f.w = field(2);
                 f.rdt = 1.0 / P.dt; f.scale = P.dx * P.dy; f.spec = FS.p;
@@ -848,7 +856,7 @@ int Ctx::autotune() {
     if (ycol_allowed() && plane_force != 0) {
         const long long l0 = launches;
         auto solve = [&]() -> int { return poisson_once((double*)p.p, 0.0, true); };
-        float tb = timeit(solve);
+        float tb = timeit(1e30f, solve);
         yfused = 1;
         int bestyf = 0;
         for (const PlaneArgs& cand : plane_candidates(nx, ny, sizeof(double2), pa)) {
@@ -857,7 +865,7 @@ int Ctx::autotune() {
                 pa = cand;
                 plans_of(pol, pa);
                 pa.batch = 1;
-                const float t = timeit(solve);
+                const float t = timeit(tb, solve);
                 if (t < tb) { tb = t; bestpa = pa; bestpol = pol; bestyf = 1; }
             }
         }
@@ -876,7 +884,7 @@ int Ctx::autotune() {
     for (int kc : kcs) {
         if (kc > nz || (long)((nz + kc - 1) / kc) * batch > 65535) continue;   // beyond the launch grid's z limit
         kchunk = kc;
-        const float t = timeit([&]() -> int {
+        const float t = timeit(bestk, [&]() -> int {
             StepArgs a{};
             a.nx = nx; a.ny = ny; a.nz = nz; a.batch = batch; a.sN = N; a.kchunk = kc;
             a.rigid = rigid; a.nonlinear = 1;
