@@ -2236,21 +2236,24 @@ static cudaError_t launch_rows_reg_t(const PlaneArgs& a, bool fwd, cudaStream_t 
     using G = RowReg<N1, N2, R>;
     const dim3 g(a.ny / G::TJ, (a.kcount ? a.kcount : a.nz) * std::max(1, a.batch));
     const size_t sm = G::elems * sizeof(cpx<R>);
-    if (a.ysplit) {
-        if (fwd && a.mode == 0) return launch_pdl(k_rows_fwd_reg<R, N1, N2, true, 0>, g, dim3(G::NT), sm, s, a);
-        if (fwd && a.mode == 1) return launch_pdl(k_rows_fwd_reg<R, N1, N2, true, 1>, g, dim3(G::NT), sm, s, a);
-        if (fwd) return launch_pdl(k_rows_fwd_reg<R, N1, N2, true, 2>, g, dim3(G::NT), sm, s, a);
-        return launch_pdl(k_rows_inv_reg<R, N1, N2, true>, g, dim3(G::NT), sm, s, a);
+    // forward: FP32 alone, a divergence or a residual one; the y-split layout:
+    // FP32 alone (Ctx::init)
+    if constexpr (sizeof(R) == 4) {
+        if (fwd && a.mode == 1) return cudaErrorInvalidValue;
+        if (a.ysplit) {
+            if (!fwd) return launch_pdl(k_rows_inv_reg<R, N1, N2, true>, g, dim3(G::NT), sm, s, a);
+            return a.mode == 0 ? launch_pdl(k_rows_fwd_reg<R, N1, N2, true, 0>, g, dim3(G::NT), sm, s, a)
+                               : launch_pdl(k_rows_fwd_reg<R, N1, N2, true, 2>, g, dim3(G::NT), sm, s, a);
+        }
+        if (fwd) return a.mode == 0 ? launch_pdl(k_rows_fwd_reg<R, N1, N2, false, 0>, g, dim3(G::NT), sm, s, a)
+                                    : launch_pdl(k_rows_fwd_reg<R, N1, N2, false, 2>, g, dim3(G::NT), sm, s, a);
     }
-    if (fwd && a.mode == 0) return launch_pdl(k_rows_fwd_reg<R, N1, N2, false, 0>, g, dim3(G::NT), sm, s, a);
-    if (fwd && a.mode == 1) return launch_pdl(k_rows_fwd_reg<R, N1, N2, false, 1>, g, dim3(G::NT), sm, s, a);
-    if (fwd) return launch_pdl(k_rows_fwd_reg<R, N1, N2, false, 2>, g, dim3(G::NT), sm, s, a);
     return launch_pdl(k_rows_inv_reg<R, N1, N2, false>, g, dim3(G::NT), sm, s, a);
 }
 // The register rows pass when nx/2 has a two-factor split, else false.  The
-// FP64 forward pass keeps the staged kernel (92.8 us for the forward transform
-// at 256x256x128, 99.0 us with the register form's 94 registers and five
-// blocks an SM).
+// FP64 forward pass has the staged kernel alone (89.1 us for the forward
+// transform at 256x256x128; a register form of it, 94 registers and five blocks
+// an SM, took 99.0).
 template <typename R>
 static bool rows_reg(const PlaneArgs& a, bool fwd, cudaStream_t s, cudaError_t* e) {
     if (fwd && sizeof(R) == 8) return false;
@@ -2263,11 +2266,14 @@ static bool rows_reg(const PlaneArgs& a, bool fwd, cudaStream_t s, cudaError_t* 
     }
 }
 
+// the sources that occur: a divergence, in FP64 a given field (projections), in
+// FP32 a residual's divergence (mixed solves)
 template <typename R, int MX>
 static cudaError_t launch_rows_fwd(const PlaneArgs& a, dim3 g, size_t sm, cudaStream_t s) {
+    constexpr int SRC = sizeof(R) == 8 ? 1 : 2;
     if (a.mode == 0) return launch_pdl(k_rows_fwd<R, MX, 0>, g, dim3(kPlaneThreads), sm, s, a);
-    if (a.mode == 1) return launch_pdl(k_rows_fwd<R, MX, 1>, g, dim3(kPlaneThreads), sm, s, a);
-    return launch_pdl(k_rows_fwd<R, MX, 2>, g, dim3(kPlaneThreads), sm, s, a);
+    if (a.mode == SRC) return launch_pdl(k_rows_fwd<R, MX, SRC>, g, dim3(kPlaneThreads), sm, s, a);
+    return cudaErrorInvalidValue;
 }
 
 template <typename R, int MX, int MY>
@@ -2358,8 +2364,9 @@ static cudaError_t setup_m() {
     if ((e = cudaFuncSetAttribute(k_plane_fwd<R, MAXR>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))) return e;
     if ((e = cudaFuncSetAttribute(k_plane_inv<R, MAXR>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))) return e;
     if ((e = cudaFuncSetAttribute(k_rows_fwd<R, MAXR, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm))) return e;
-    if ((e = cudaFuncSetAttribute(k_rows_fwd<R, MAXR, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm))) return e;
-    if ((e = cudaFuncSetAttribute(k_rows_fwd<R, MAXR, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm))) return e;
+    if ((e = cudaFuncSetAttribute(k_rows_fwd<R, MAXR, sizeof(R) == 8 ? 1 : 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  maxsm)))
+        return e;
     if ((e = cudaFuncSetAttribute(k_rows_inv<R, MAXR>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm))) return e;
     if ((e = cudaFuncSetAttribute(k_ylines<R, MAXR>, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm))) return e;
     if ((e = max_dynamic_smem(k_rows_fwd_pipe<R, MAXR>))) return e;
@@ -2371,21 +2378,30 @@ static cudaError_t setup_t() {
     if ((e = max_dynamic_smem(k_ylines_reg<R, 8, 8>))) return e;
     if ((e = max_dynamic_smem(k_ylines_reg<R, 16, 8>))) return e;
     if ((e = max_dynamic_smem(k_ylines_reg<R, 16, 16>))) return e;
-#define PS3D_ROWS_SETUP(YS)                                                   \
-    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 8, 8, YS, 0>))) return e;     \
-    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 8, 8, YS, 1>))) return e;     \
-    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 8, 8, YS, 2>))) return e;     \
-    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 16, 8, YS, 0>))) return e;    \
-    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 16, 8, YS, 1>))) return e;    \
-    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 16, 8, YS, 2>))) return e;    \
-    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 16, 16, YS, 0>))) return e;   \
-    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 16, 16, YS, 1>))) return e;   \
-    if ((e = max_dynamic_smem(k_rows_fwd_reg<R, 16, 16, YS, 2>))) return e;   \
-    if ((e = max_dynamic_smem(k_rows_inv_reg<R, 8, 8, YS>))) return e;       \
-    if ((e = max_dynamic_smem(k_rows_inv_reg<R, 16, 8, YS>))) return e;      \
-    if ((e = max_dynamic_smem(k_rows_inv_reg<R, 16, 16, YS>))) return e;
-    PS3D_ROWS_SETUP(false)
-    PS3D_ROWS_SETUP(true)
+#define PS3D_ROWS_SETUP(K)                                 \
+    if ((e = max_dynamic_smem(K(8, 8)))) return e;         \
+    if ((e = max_dynamic_smem(K(16, 8)))) return e;        \
+    if ((e = max_dynamic_smem(K(16, 16)))) return e;
+#define PS3D_K(N1, N2) k_rows_inv_reg<R, N1, N2, false>
+    PS3D_ROWS_SETUP(PS3D_K)
+#undef PS3D_K
+    if constexpr (sizeof(R) == 4) {
+#define PS3D_K(N1, N2) k_rows_inv_reg<R, N1, N2, true>
+        PS3D_ROWS_SETUP(PS3D_K)
+#undef PS3D_K
+#define PS3D_K(N1, N2) k_rows_fwd_reg<R, N1, N2, false, 0>
+        PS3D_ROWS_SETUP(PS3D_K)
+#undef PS3D_K
+#define PS3D_K(N1, N2) k_rows_fwd_reg<R, N1, N2, false, 2>
+        PS3D_ROWS_SETUP(PS3D_K)
+#undef PS3D_K
+#define PS3D_K(N1, N2) k_rows_fwd_reg<R, N1, N2, true, 0>
+        PS3D_ROWS_SETUP(PS3D_K)
+#undef PS3D_K
+#define PS3D_K(N1, N2) k_rows_fwd_reg<R, N1, N2, true, 2>
+        PS3D_ROWS_SETUP(PS3D_K)
+#undef PS3D_K
+    }
 #undef PS3D_ROWS_SETUP
     if ((e = cudaFuncSetAttribute(k_zsolve<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024))) return e;
     if ((e = max_dynamic_smem(k_thomas2<R, false, false>))) return e;
