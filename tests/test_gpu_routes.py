@@ -4,13 +4,37 @@ import numpy as np
 import pytest
 
 from ps3d_b200 import abi
+from ps3d_b200 import configs as cf
 from ps3d_b200.model import Model
 from ps3d_b200.serve import Server, request
 from oracle.binding import Oracle
-from tests.helpers import FIELDS, compare_state, load_oracle, random_state, small_params
+from tests.helpers import (FIELDS, compare_state, load_oracle, random_state, small_params, smooth_state,
+                           upload_from_oracle)
 
 pytestmark = pytest.mark.gpu
-TOL_KERNEL = 1e-12   # one FP64 pressure solve
+TOL_KERNEL = 1e-12   # one FP64 pressure solve or projection
+TOL64 = 1e-11        # several FP64 steps: the suite's bound for rounding in another order
+TOL_MIXED = 1e-5     # the mixed path
+
+
+def _pair(p, f):
+    o, m = Oracle(p), Model(p)
+    load_oracle(o, f)
+    upload_from_oracle(m, o)
+    return o, m
+
+
+def _projected(o, m, p, tol):
+    """One pressure solve against the oracle; a velocity carries p's rounding
+    times dt over its grid distance."""
+    o.pressure_solver()
+    m.pressure_solver()
+    got = m.download(tendencies=False)
+    pn = np.linalg.norm(cf.interior(o.field("p")))
+    for k, d in (("p", None), ("u", p.dx), ("v", p.dy), ("w", p.dz)):
+        want = cf.interior(o.field(k))
+        t = tol * np.linalg.norm(want) + (8 * np.finfo(float).eps * p.dt / d * pn if d else 0.0)
+        assert np.linalg.norm(cf.interior(got[k]) - want) <= t, (k, np.linalg.norm(cf.interior(got[k]) - want), t)
 
 
 @pytest.mark.parametrize("n", [(128, 16, 8), (96, 20, 10)])
@@ -55,3 +79,67 @@ def test_pinned_fused_solve(pin, fused, monkeypatch):
     assert f"yfused={fused}" in m.describe() and "tuned=pinned" in m.describe()
     err = compare_state(m, o)
     assert max(err.values()) < TOL_KERNEL, err
+
+
+@pytest.mark.parametrize("form", ["fused", "0", "2", "3"])
+@pytest.mark.parametrize("impl", ["0", "1"])
+@pytest.mark.parametrize("nz", [3, 16, 41])
+def test_columns_without_a_wavenumber(nz, impl, form, monkeypatch):
+    """Lx = nx dx / 2 and Ly = ny dy / 2: besides (0,0), the columns at kx =
+    nx/2, at ky = ny/2 and at both have no horizontal wavenumber, and the
+    vertical solve takes them by the (0,0) recurrence, part by part."""
+    if form == "fused" and impl == "0":
+        pytest.skip("the cluster kernels transform along y themselves")
+    monkeypatch.setenv("PS3D_AUTOTUNE", "0")
+    monkeypatch.setenv("PS3D_PLANE_IMPL", impl)
+    monkeypatch.setenv("PS3D_YFUSED", "1" if form == "fused" else "0")
+    if form != "fused":
+        monkeypatch.setenv("PS3D_THOMAS_FORM", form)
+    p = small_params(16, 12, nz, rigid=True, dx=2 * 32e3 / 16, dy=2 * 32e3 / 12)
+    o, m = _pair(p, random_state(p, seed=52))
+    assert f"yfused={int(form == 'fused')}" in m.describe()
+    _projected(o, m, p, TOL_KERNEL)
+
+
+@pytest.mark.parametrize("n", [(18, 10, 64), (20, 6, 128), (20, 6, 50)])
+def test_periodic_solve_mixed(n):
+    """The periodic solve on FP32 spectra, in registers and staged."""
+    p = small_params(*n, rigid=False)
+    f = random_state(p, seed=54)
+    o = Oracle(p)
+    load_oracle(o, f)
+    p.precision = abi.PS3D_MIXED
+    m = Model(p)
+    m.upload(**{k: f[k] for k in FIELDS})
+    _projected(o, m, p, TOL_MIXED)
+
+
+@pytest.mark.parametrize("mode", [abi.PS3D_PROJ_NORMAL_MODE, abi.PS3D_PROJ_EXCHANGE])
+@pytest.mark.parametrize("n", [(18, 10, 32), (12, 10, 64), (10, 6, 128), (8, 6, 256)])
+def test_periodic_projection_in_registers(n, mode):
+    """The forward-only and inverse-only z transforms on columns in registers,
+    with a last block that is not full."""
+    p = small_params(*n, rigid=False, Lz=1000.0 * n[2] / 16)
+    o, m = _pair(p, smooth_state(p, seed=55))
+    if mode == abi.PS3D_PROJ_EXCHANGE:
+        o.project(abi.PS3D_PROJ_BASE_POINT)
+        m.project(abi.PS3D_PROJ_BASE_POINT)
+    o.project(mode)
+    m.project(mode)
+    err = compare_state(m, o, names=FIELDS)
+    assert max(err.values()) < TOL_KERNEL, err
+
+
+@pytest.mark.parametrize("harmonic", [False, True])
+@pytest.mark.parametrize("n", [(64, 64, 23), (64, 128, 23), (64, 180, 23), (256, 256, 5), (64, 128, 20)])
+def test_biharmonic_friction_marches(n, harmonic):
+    """Biharmonic friction on grids where a block of its kernel (two an SM)
+    marches over chunks of 2, 3, 4 and 5 levels, the last one shorter or
+    with the lid in it; nz = 20: triply periodic."""
+    p = small_params(*n, rigid=n[2] != 20, Ahbi=1e7, Avbi=1e1, Khbi=1e7, Kvbi=1e1,
+                     **({} if harmonic else dict(Ah=0.0, Av=0.0)))
+    o, m = _pair(p, smooth_state(p, seed=56))
+    o.integrate(3)
+    m.run(3)
+    err = compare_state(m, o)
+    assert max(err.values()) < TOL64, err
