@@ -364,7 +364,10 @@ PS3D_API int ps3d_slab_create(const ps3d_params* global, int nranks, int rank, i
     c.win_kbeg = 1; c.win_kcount = s->nzl; c.win_kofs = s->k0 - 1; c.win_nzg = s->nzg;
     int rc = c.init(lp, device);
     if (rc) return rc;
-    if ((s->mixed ? c.pa32 : c.pa64).impl != 1) return PS3D_ERR_UNSUPPORTED;   // grid the rows + y-lines kernels cannot take
+    // grids that the rows + y-lines kernels take in runs of at least 8 rows (ny
+    // a multiple of 8); the shorter runs serve whole grids alone
+    const ps3d::PlaneArgs& pa = s->mixed ? c.pa32 : c.pa64;
+    if (pa.impl != 1 || pa.tj < 8) return PS3D_ERR_UNSUPPORTED;
     c.use_graphs = false;
     if (!rigid) {
         // the global z transform and its wavenumbers (my_fft.f90:87-156)

@@ -5,8 +5,9 @@ import pytest
 
 from ps3d_b200 import abi
 from ps3d_b200 import configs as cf
-from ps3d_b200.model import Model
+from ps3d_b200.model import Model, PS3DError
 from ps3d_b200.serve import Server, request
+from ps3d_b200.slab import Slab
 from oracle.binding import Oracle
 from tests.helpers import (FIELDS, compare_state, load_oracle, random_state, small_params, smooth_state,
                            upload_from_oracle)
@@ -143,3 +144,18 @@ def test_biharmonic_friction_marches(n, harmonic):
     m.run(3)
     err = compare_state(m, o)
     assert max(err.values()) < TOL64, err
+
+
+@pytest.mark.parametrize("ny,taken", [(2, False), (4, False), (10, False), (36, False), (8, True), (24, True)])
+@pytest.mark.parametrize("precision", [abi.PS3D_FP64, abi.PS3D_MIXED])
+def test_slabs_take_rows_in_eights(ny, taken, precision):
+    """z-slabs exist for grids whose ny is a multiple of 8 and are refused for
+    others, which whole grids take in shorter runs of rows."""
+    p = small_params(16, ny, 8, rigid=True, precision=precision)
+    Model(p).close()
+    if taken:
+        Slab(p, 2, 0).close()
+    else:
+        with pytest.raises(PS3DError) as e:
+            Slab(p, 2, 0)
+        assert e.value.status == abi.PS3D_ERR_UNSUPPORTED
