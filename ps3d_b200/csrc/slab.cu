@@ -465,7 +465,7 @@ PS3D_API int ps3d_slab_upload(ps3d_slab* s, const double* u, const double* v, co
 static int apply_pending(ps3d_slab* s) {
     Ctx& c = *s->ctx;
     if (c.pending) {
-        CK(ps3d::launch_correct(c.field(0), c.field(1), c.field(2), c.pcor, c.nx, c.ny, c.nz, 1, c.dtp,
+        CK(ps3d::launch_correct(c.field(0), c.field(1), c.field(2), c.pcor, c.nx, c.ny, c.nz, s->rigid, c.dtp,
                                 c.dtp / c.P.dsqr, 1.0 / c.P.dx, 1.0 / c.P.dy, 1.0 / c.P.dz, c.stream, 1, 0, s->nzl + 2,
                                 s->k0 - 1, s->nzg));
         c.pending = false;

@@ -7,7 +7,7 @@ from ps3d_b200 import abi
 from ps3d_b200 import configs as cf
 from ps3d_b200.model import Model, PS3DError
 from ps3d_b200.serve import Server, request
-from ps3d_b200.slab import Slab
+from ps3d_b200.slab import Slab, SlabGroup
 from oracle.binding import Oracle
 from tests.helpers import (FIELDS, compare_state, load_oracle, random_state, small_params, smooth_state,
                            upload_from_oracle)
@@ -159,3 +159,23 @@ def test_slabs_take_rows_in_eights(ny, taken, precision):
         with pytest.raises(PS3DError) as e:
             Slab(p, 2, 0)
         assert e.value.status == abi.PS3D_ERR_UNSUPPORTED
+
+
+@pytest.mark.parametrize("rigid", [True, False])
+def test_slab_download_in_mid_run(rigid, monkeypatch):
+    """Every level of a slab run, w at the top one included, is the single
+    grid's, at a download between steps and after further steps."""
+    monkeypatch.setenv("PS3D_PLANE_IMPL", "1")
+    p = small_params(16, 8, 20, rigid=rigid, Lz=1250.0)
+    f = random_state(p, seed=58)
+    m, s = Model(p), SlabGroup(p, 2)
+    m.upload(**{k: f[k] for k in FIELDS})
+    s.upload(*[np.ascontiguousarray(cf.interior(f[k])) for k in FIELDS])
+    for n in (2, 3):
+        m.run(n)
+        s.step(n)
+        ref, got = m.download(tendencies=False), s.download()
+        for k in FIELDS + ("p",):
+            want = cf.interior(ref[k])
+            assert np.linalg.norm(got[k] - want) < TOL64 * np.linalg.norm(want), (n, k)
+    s.close()
