@@ -154,14 +154,16 @@ int slab_forward(ps3d_slab* s) {
     CK(ps3d::launch_plane_fwd(a, s->mixed, c.stream));
     const size_t es = s->es();
     for (int r = 0; r < s->nranks; ++r)
-        CK(cudaMemcpy2DAsync((char*)s->xbuf + (size_t)s->nzl * s->cbeg[r] * es, s->ccnt[r] * es,
-                             (const char*)c.FS.p + s->cbeg[r] * es, s->ncols * es, s->ccnt[r] * es, s->nzl,
-                             cudaMemcpyDeviceToDevice, c.stream));
+        if (s->ccnt[r])
+            CK(cudaMemcpy2DAsync((char*)s->xbuf + (size_t)s->nzl * s->cbeg[r] * es, s->ccnt[r] * es,
+                                 (const char*)c.FS.p + s->cbeg[r] * es, s->ncols * es, s->ccnt[r] * es, s->nzl,
+                                 cudaMemcpyDeviceToDevice, c.stream));
     return PS3D_OK;
 }
 
 int slab_vsolve(ps3d_slab* s) {
     Ctx& c = *s->ctx;
+    if (!s->ccnt[s->rank]) return PS3D_OK;   // more ranks than columns: none here (to the solves 0 means the whole grid)
     ps3d::ColumnArgs a{};
     a.nx = c.nx; a.ny = c.ny; a.nz = s->nzg; a.nxh = c.nxh;
     a.spec = s->colbuf;
@@ -186,9 +188,10 @@ int slab_inverse(ps3d_slab* s) {
     Ctx& c = *s->ctx;
     const size_t es = s->es();
     for (int r = 0; r < s->nranks; ++r)
-        CK(cudaMemcpy2DAsync((char*)c.FS.p + s->cbeg[r] * es, s->ncols * es,
-                             (const char*)s->xbuf + (size_t)s->nzl * s->cbeg[r] * es, s->ccnt[r] * es,
-                             s->ccnt[r] * es, s->nzl, cudaMemcpyDeviceToDevice, c.stream));
+        if (s->ccnt[r])
+            CK(cudaMemcpy2DAsync((char*)c.FS.p + s->cbeg[r] * es, s->ncols * es,
+                                 (const char*)s->xbuf + (size_t)s->nzl * s->cbeg[r] * es, s->ccnt[r] * es,
+                                 s->ccnt[r] * es, s->nzl, cudaMemcpyDeviceToDevice, c.stream));
     ps3d::PlaneArgs b = window(s, s->mixed ? c.pa32 : c.pa64);
     b.spec = c.FS.p;
     b.out = (double*)c.p.p;

@@ -179,3 +179,23 @@ def test_slab_download_in_mid_run(rigid, monkeypatch):
             want = cf.interior(ref[k])
             assert np.linalg.norm(got[k] - want) < TOL64 * np.linalg.norm(want), (n, k)
     s.close()
+
+
+@pytest.mark.parametrize("rigid", [True, False])
+def test_slabs_without_columns(rigid, monkeypatch):
+    """More ranks than spectral columns: some slabs hold none and solve none."""
+    monkeypatch.setenv("PS3D_PLANE_IMPL", "1")
+    p = small_params(2, 8, 40, rigid=rigid, Lz=2500.0)   # 16 columns
+    f = random_state(p, seed=57)
+    m = Model(p)
+    m.upload(**{k: f[k] for k in FIELDS})
+    m.run(3)
+    ref = m.download(tendencies=False)
+    s = SlabGroup(p, 20)
+    s.upload(*[np.ascontiguousarray(cf.interior(f[k])) for k in FIELDS])
+    s.step(3)
+    got = s.download()
+    s.close()
+    for k in FIELDS + ("p",):
+        want = cf.interior(ref[k])
+        assert np.linalg.norm(got[k] - want) < TOL64 * np.linalg.norm(want), k
