@@ -334,10 +334,11 @@ PS3D_API int ps3d_ensemble_info(ps3d_ensemble* e, int* ngroups, long long* launc
  * (PACK_STATE, exchange, UNPACK_STATE).  ps3d_slab_group_step does all of it
  * for the ranks of one process (device copies; one GPU or several).
  * Upload/download take the rank's interior levels, [nzl][ny][nx] doubles,
- * x fastest (no halos).  Rigid lid or triply periodic, the fused step
- * (Laplacian friction, wavemaker and background-flow forcing; not
- * biharmonic friction, a host callback, or background flow together with
- * Laplacian friction: PS3D_ERR_UNSUPPORTED).                               */
+ * x fastest (no halos).  ny a multiple of 8 (else PS3D_ERR_UNSUPPORTED),
+ * rigid lid or triply periodic, the fused step (Laplacian friction,
+ * wavemaker and background-flow forcing; not biharmonic friction, a host
+ * callback, or background flow together with Laplacian friction:
+ * PS3D_ERR_UNSUPPORTED).                                                   */
 #define PS3D_SLAB_TENDENCY     0
 #define PS3D_SLAB_PACK_STATE   1
 #define PS3D_SLAB_UNPACK_STATE 2

@@ -113,8 +113,8 @@ __device__ __forceinline__ double2 plane_source_pair(const PlaneArgs& a, const d
 // are found once.  LB rows' loads go out together; store(r, d) takes row j0+r.
 // Formed point by point, 157 of a pair's 272 instructions in the rows pass were
 // index arithmetic; forward transforms, before and after: 256x256x128 FP64 99.4
-// and 92.5 us, 512x256x64 94.4 and 86.6 us mixed, 128x128x64 25.5 and 20.0 us
-// mixed.  LB is chosen against registers: two rows in flight in FP64 (four
+// and 92.5 us (89 with the blocks of rows_blocks), 512x256x64 94.4 and 86.6 us
+// mixed, 128x128x64 25.5 and 20.0 us mixed.  LB is chosen against registers: two rows in flight in FP64 (four
 // spill, 117 us), one with the pressure's
 // seven further loads (two cost the FP32 register pass blocks: 108.9 against
 // 86.6 us at 512x256x64), two where a thread walks only 8 rows (nx = 128).
@@ -1368,7 +1368,7 @@ cudaError_t launch_colsolve(const PlaneArgs& p, const ColumnArgs& c, cudaStream_
 constexpr int kZLines = 32;
 
 // Columns staged in shared memory, any length that factors: a lane keeps one
-// column, so no index is divided (256x256x96 FP64 92 -> 59 us, FP32 90 -> 51).
+// column, so no index is divided (256x256x96 FP64 102 -> 64 us, FP32 100 -> 48).
 template <typename R>
 __global__ void __launch_bounds__(256, 2) k_zsolve(const ColumnArgs a) {
     pdl_trigger();
@@ -1438,7 +1438,7 @@ __global__ void __launch_bounds__(256, 2) k_zsolve(const ColumnArgs a) {
 // the same bits in FP32.
 // Bound by its FP64 arithmetic and two block barriers at four blocks an SM:
 // 512x256x128 78 us FP64 (270 MB, 54 % of the copy bandwidth) and 56 us FP32,
-// where the staged kernel with divided indices took 224 and 199 us.
+// where the staged kernel takes 128 and 82 us (with divided indices 224 and 199).
 constexpr int kZRegThreads = 128;
 
 template <typename R, int N1>
@@ -2251,9 +2251,9 @@ static cudaError_t launch_rows_reg_t(const PlaneArgs& a, bool fwd, cudaStream_t 
     return launch_pdl(k_rows_inv_reg<R, N1, N2, false>, g, dim3(G::NT), sm, s, a);
 }
 // The register rows pass when nx/2 has a two-factor split, else false.  The
-// FP64 forward pass has the staged kernel alone (89.1 us for the forward
+// FP64 forward pass has the staged kernel alone (89 us for the forward
 // transform at 256x256x128; a register form of it, 94 registers and five blocks
-// an SM, took 99.0).
+// an SM, took 99).
 template <typename R>
 static bool rows_reg(const PlaneArgs& a, bool fwd, cudaStream_t s, cudaError_t* e) {
     if (fwd && sizeof(R) == 8) return false;
@@ -2553,9 +2553,9 @@ bool zsolve_fits(int nz, bool fp32) {
     return zsolve_smem(nz, fp32 ? sizeof(float2) : sizeof(double2)) <= 227 * 1024;
 }
 
-// Columns in registers where the plan's radices are {16, N1}: nz = 32 (9.8 us
-// at 64x66x32x3, staged 13.6), 64 (11.4, 16.0 at 128x64), 128 (80, 206 at
-// 512x256), 256 (11.8, 40.6 at 32x32).  Every other length is staged
+// Columns in registers where the plan's radices are {16, N1}, FP64 against the
+// staged kernel: nz = 32 (10.6 and 11.1 us at 64x64), 64 (12.8 and 14.9 at
+// 128x64), 128 (78 and 128 at 512x256), 256 (18.7 and 27.7 at 64x64).  Every other length is staged
 // (PS3D_ZSOLVE=0 stages all).
 template <typename R, int N1>
 static cudaError_t launch_zsolve_reg(const ColumnArgs& a, cudaStream_t s) {

@@ -22,8 +22,8 @@
 // Each state word is read once from HBM and each tendency and new value is
 // written once.
 //
-// What bounds it: HBM.  At 256x256x128 it runs 237 us in FP64 (168 B a point,
-// 5.9 TB/s) and 222-231 us in the mixed form (132 B, 4.9 TB/s).  The form it
+// What bounds it: HBM.  At 256x256x128 it runs 240 us in FP64 (168 B a point,
+// 5.9 TB/s) and 210 us in the mixed form (132 B, 5.3 TB/s).  The form it
 // replaced (one point a thread, planes loaded through registers behind two
 // barriers a level, all fluxes formed from shared memory) took 321 and 292 us:
 // it kept the L1/shared data path at 72 % with 257 wavefronts and 632
@@ -488,9 +488,9 @@ __device__ __forceinline__ void step_tile(const StepArgs& a, int kchunk, int bx,
 }
 
 // Blocks an SM the step kernels are built for: the plain and the u, v, w
-// friction forms fit 168 registers without a spill and run three (247 us FP64,
-// 224-234 us mixed at 256x256x128; held to two 270 and 254 us), the others
-// would spill and run two.
+// friction forms fit 168 registers without a spill and run three (held to two
+// they took 9 % longer in FP64 and 11 % mixed at 256x256x128), the others would
+// spill and run two.
 constexpr int step_blocks(int harm, bool wm, bool bg) { return harm > 1 || wm || bg ? 2 : 3; }
 
 template <typename TT, int BY, int HARM, bool WM, bool BG>
